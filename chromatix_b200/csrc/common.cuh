@@ -31,11 +31,16 @@ __host__ __device__ __forceinline__ int add_mod(int n, int s, int m) {
 // fftfreq numerator of FFT bin k for length n (numpy/jax convention).
 __host__ __device__ __forceinline__ int freq_index(int k, int n) { return k < (n + 1) / 2 ? k : k - n; }
 
-// Reduce an FP64 phase to [-pi, pi] before the FP32 sin/cos.
+// Reduce an FP64 phase to [-pi, pi] before the FP32 sin/cos.  The number of
+// turns is rounded by adding and subtracting 1.5 2^52 (exact for |turns| <
+// 2^51, far past any phase with a meaning): two FP64 additions instead of a
+// rounding conversion, which runs at an eighth of their rate.
 __device__ __forceinline__ float reduce_phase(double ph) {
   const double inv2pi = 0.15915494309189533576888376337251;
   const double twopi = 6.283185307179586476925286766559;
-  return (float)(ph - twopi * rint(ph * inv2pi));
+  const double magic = 6755399441055744.0;
+  const double turns = __dadd_rn(__dadd_rn(ph * inv2pi, magic), -magic);
+  return (float)(ph - twopi * turns);
 }
 
 // exp(i ph) for an FP64 phase: exact reduction to [-pi, pi] in FP64, then the

@@ -527,20 +527,6 @@ __host__ __device__ constexpr unsigned edge_zero_mask() {
   return m;
 }
 
-// First-stage zero mask for an input that is nonzero only on the central
-// band [N / 4, 3 N / 4) (a field zero-padded to twice its size on both
-// sides): with a first radix R_0 divisible by 4, the inputs j + r N / R_0 with
-// r < R_0 / 4 or r >= 3 R_0 / 4 are zero.  0 (no mask) otherwise.
-template <int N>
-__host__ __device__ constexpr unsigned center_band_mask() {
-  constexpr int R0 = Plan<N>::P.r[0];
-  unsigned m = 0u;
-  if (R0 % 4 == 0)
-    for (int r = 0; r < R0; ++r)
-      if (r < R0 / 4 || r >= 3 * R0 / 4) m |= 1u << r;
-  return m;
-}
-
 // First-stage zero mask for an input that is nonzero only on [0, N / 2)
 // (zero padding to twice the length): with an even first radix R_0 the
 // inputs r >= R_0 / 2 of every first-stage butterfly (indices

@@ -33,9 +33,11 @@ void set_error(const char* fmt, ...);
   } while (0)
 
 // FFT lengths compiled into the fast path: 2^a, 3 * 2^a, 5 * 2^a, 7 * 2^a up to 4096.
-#define CX_FOR_EACH_SIZE(X)                                                                          \
+#define CX_FOR_EACH_SHORT_SIZE(X)                                                                    \
   X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(10) X(12) X(14) X(16) X(20) X(24) X(28) X(32) X(40) X(48)    \
-  X(56) X(64) X(80) X(96) X(112) X(128) X(160) X(192) X(224) X(256) X(320) X(384) X(448) X(512)    \
+  X(56) X(64) X(80) X(96) X(112)
+#define CX_FOR_EACH_SIZE(X)                                                                          \
+  CX_FOR_EACH_SHORT_SIZE(X) X(128) X(160) X(192) X(224) X(256) X(320) X(384) X(448) X(512)    \
   X(640) X(768) X(896) X(1024) X(1280) X(1536) X(1792) X(2048) X(2560) X(3072) X(3584) X(4096)
 
 // Longer lengths compiled only for the 1D transform (cx_fft1d) and the

@@ -4,7 +4,9 @@
 // asm_propagate), 355-394 (kernel_propagate FFT branch), 466-580
 // (compute_transfer_propagator, compute_asm_propagator).
 //
-// Three passes over the padded (py, px) grid:
+// Three passes over the padded (py, px) grid (lengths of 128 and more run them
+// on pairs of rows and columns, prop2d_pair.cuh; the kernels here take the
+// shorter ones):
 //   A  row FFT of the ny input rows, zero padding done in the loader
 //      (rows outside the data are never materialised);
 //   B  per V-column tile: column FFT -> x H(ky, kx) evaluated on the fly ->
@@ -210,20 +212,22 @@ __device__ __forceinline__ PropK prop_consts(const Prop2DArgs& a, const cx_plane
   return c;
 }
 
-// sqrt(x) for 0 <= x <= 1 to FP64 accuracy from the FP32 hardware estimate
-// and one Newton-Raphson (Heron) step in FP64:
-//   s0 = x_f rsqrt(x_f),  s1 = s0 + (x - s0^2) / (2 s0),
-// with 1 / s0 taken from the same FP32 reciprocal square root.  s0 carries
-// a relative error e ~ 1e-7, so s1 is within ~e^2 + e * |x - s0^2| / s0 ~ 1e-14
-// of sqrt(x) relatively (the ASM phase K sqrt(.) with K <= 1e5 rad then stays
-// within 1e-9 rad).  x below the smallest normal float gives 0 (its root,
-// < 1e-19, times K is far below the phase budget).
+// sqrt(x) for 0 <= x <= 1 to FP64 accuracy from the hardware's FP64 reciprocal
+// square root estimate r and two Heron steps,
+//   s <- s + (x - s^2) r / 2,  s_0 = x r.
+// r carries a relative error e < 2^-19, so the steps leave e^2 and e^3
+// relatively (the ASM phase K sqrt(.) with K <= 1e5 rad stays within 1e-9 rad).
+// No conversion between FP64 and FP32 (those run at an eighth of the FP64
+// rate).  x below the smallest normal float gives 0 (its root, < 1e-19, times
+// K is far below the phase budget).
 __device__ __forceinline__ double sqrt_unit_f64(double x) {
-  const float xf = (float)x;
-  if (!(xf > 0.f)) return 0.0;
-  const float r = rsqrtf(xf);
-  const double s0 = (double)(xf * r);
-  return fma(fma(-s0, s0, x), 0.5 * (double)r, s0);
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double h = 0.5 * r;
+  double s = x * r;
+  s = fma(fma(-s, s, x), h, s);
+  s = fma(fma(-s, s, x), h, s);
+  return x > 1.2e-38 ? s : 0.0;
 }
 
 // prop_kernel_accurate for the transfer and ASM kinds with the per-plane
@@ -322,53 +326,65 @@ __device__ __forceinline__ PropCol prop_col(const Prop2DArgs& a, const cx_plane&
   return pc;
 }
 
-__device__ __forceinline__ float2 prop_col_h(int ky, int kx, const PropCol& pc, const Prop2DArgs& a,
-                                             const cx_plane& pl, const PropK& c) {
+// mode MODE's value at frequency number kf (= freq_index(ky)) of the column
+template <int MODE>
+__device__ __forceinline__ float2 prop_col_at(double kf, int ky, int kx, const PropCol& pc, const Prop2DArgs& a,
+                                              const cx_plane& pl, const PropK& c) {
   const double pi = 3.141592653589793238462643383279502884;
-  const double fy = (double)freq_index(ky, a.py) * c.iy;
+  const double fy = kf * c.iy;
   const double gy = fy - a.ky0;
-  switch (pc.mode) {
-    case 1: {
-      const double kern = 1.0 - c.q2 * (gy * gy + pc.gx2);
-      const double sh = c.shifted ? 2.0 * pi * (fy * pl.shift_y + pc.fx * pl.shift_x) : 0.0;
-      double amp = 1.0, ph = sh;
-      if (kern >= 0.0 || a.remove_evanescent)
-        ph += c.K * sqrt_unit_f64(kern);
-      else
-        amp = exp(-c.K * sqrt_unit_f64(-kern));
-      const float2 e = expi_reduced(ph);
-      return make_float2((float)amp * e.x, (float)amp * pc.sgn * e.y);
-    }
-    case 2: {
-      const float2 e = expi_reduced(c.tz * (gy * gy + pc.gx2));
+  if constexpr (MODE == 1) {
+    const double kern = 1.0 - c.q2 * (gy * gy + pc.gx2);
+    const double sh = c.shifted ? 2.0 * pi * (fy * pl.shift_y + pc.fx * pl.shift_x) : 0.0;
+    if (kern >= 0.0 || a.remove_evanescent) {
+      const float2 e = expi_reduced(sh + c.K * sqrt_unit_f64(kern));
       return make_float2(e.x, pc.sgn * e.y);
     }
-    case 3: {
-      const float kern = (float)(1.0 - c.q2 * (gy * gy + pc.gx2));
-      float amp = 1.f, ph = 0.f;
-      if (kern >= 0.f || a.remove_evanescent)
-        ph = (float)c.K * sqrtf(fmaxf(kern, 0.f));
-      else
-        amp = __expf(-(float)c.K * sqrtf(-kern));
-      float sn, cs;
-      __sincosf(ph - 6.2831853071795865f * rintf(ph * 0.15915494309189534f), &sn, &cs);
-      return make_float2(amp * cs, amp * pc.sgn * sn);
-    }
-    case 4: {
-      const float2 h = a.H[((size_t)pl.h_plane * a.py + ky) * a.px + kx];
-      return make_float2(h.x, pc.sgn * h.y);
-    }
+    const float amp = (float)exp(-c.K * sqrt_unit_f64(-kern));
+    const float2 e = expi_reduced(sh);
+    return make_float2(amp * e.x, amp * pc.sgn * e.y);
+  } else if constexpr (MODE == 2) {
+    const float2 e = expi_reduced(c.tz * (gy * gy + pc.gx2));
+    return make_float2(e.x, pc.sgn * e.y);
+  } else if constexpr (MODE == 3) {
+    const float kern = (float)(1.0 - c.q2 * (gy * gy + pc.gx2));
+    float amp = 1.f, ph = 0.f;
+    if (kern >= 0.f || a.remove_evanescent)
+      ph = (float)c.K * sqrtf(fmaxf(kern, 0.f));
+    else
+      amp = __expf(-(float)c.K * sqrtf(-kern));
+    float sn, cs;
+    __sincosf(ph - 6.2831853071795865f * rintf(ph * 0.15915494309189534f), &sn, &cs);
+    return make_float2(amp * cs, amp * pc.sgn * sn);
+  } else if constexpr (MODE == 4) {
+    const float2 h = a.H[((size_t)pl.h_plane * a.py + ky) * a.px + kx];
+    return make_float2(h.x, pc.sgn * h.y);
+  } else {
+    return prop_kernel_k(ky, kx, a, pl, c);
+  }
+}
+
+__device__ __forceinline__ float2 prop_col_h(int ky, int kx, const PropCol& pc, const Prop2DArgs& a,
+                                             const cx_plane& pl, const PropK& c) {
+  const double kf = (double)freq_index(ky, a.py);
+  switch (pc.mode) {
+    case 1:
+      return prop_col_at<1>(kf, ky, kx, pc, a, pl, c);
+    case 2:
+      return prop_col_at<2>(kf, ky, kx, pc, a, pl, c);
+    case 3:
+      return prop_col_at<3>(kf, ky, kx, pc, a, pl, c);
+    case 4:
+      return prop_col_at<4>(kf, ky, kx, pc, a, pl, c);
     default:
-      return prop_kernel_k(ky, kx, a, pl, c);
+      return prop_col_at<0>(kf, ky, kx, pc, a, pl, c);
   }
 }
 
 // --------------------------------------------------------------------------
 // pass A: forward row FFT with zero padding in the loader
 // --------------------------------------------------------------------------
-// BAND: the data columns lie in [NX / 4, 3 NX / 4) (checked on the host), so
-// the first stage skips the zero padding outside that band (center_band_mask)
-template <int NX, bool BAND = false>
+template <int NX>
 __global__ void __launch_bounds__(RowCfg<NX>::THREADS, RowCfg<NX>::MINB) k_prop_rows_fwd(const float2* __restrict__ u,
                                                                       float2* __restrict__ T, Prop2DArgs a) {
   using C = RowCfg<NX>;
@@ -395,15 +411,13 @@ __global__ void __launch_bounds__(RowCfg<NX>::THREADS, RowCfg<NX>::MINB) k_prop_
     auto store = [&](int k, float2 v, int) {
       if (valid) dst[k] = v;
     };
-    team_fft<NX, false, Plan<NX>::LPV, false, (BAND ? center_band_mask<NX>() : 0u)>(s, tw, lane, team, load, store);
+    team_fft<NX, false>(s, tw, lane, team, load, store);
   }
 }
 
 // --------------------------------------------------------------------------
 // pass B: column FFT -> x H -> column IFFT on V-column tiles
 // --------------------------------------------------------------------------
-// BAND: the data rows lie in [NY / 4, 3 NY / 4) of the padded column (checked
-// on the host), so the forward transform's first stage skips the padding.
 // HT: the propagator is a table (CX_KERNEL_EXPLICIT without NA mask, e.g. the
 // multislice slice propagator): the tile's V columns of H are copied into
 // shared memory (cp.async) together with the data tile, instead of being read
@@ -411,10 +425,9 @@ __global__ void __launch_bounds__(RowCfg<NX>::THREADS, RowCfg<NX>::MINB) k_prop_
 template <int NY>
 struct PropColHt {
   static constexpr size_t SMEM = ColCfg<NY>::SMEM + sizeof(float2) * (size_t)ColCfg<NY>::V * NY;
-  static constexpr bool FITS = SMEM <= 227 * 1024;
 };
 
-template <int NY, bool BAND = false, bool HT = false>
+template <int NY, bool HT = false>
 __global__ void __launch_bounds__(ColCfg<NY>::THREADS, ColCfg<NY>::MINB) k_prop_cols(const float2* __restrict__ T,
                                                                   float2* __restrict__ T2, Prop2DArgs a) {
   using C = ColCfg<NY>;
@@ -464,8 +477,7 @@ __global__ void __launch_bounds__(ColCfg<NY>::THREADS, ColCfg<NY>::MINB) k_prop_
         s[pad_idx(k)] = valid ? cmul(v, prop_col_h(k, kx, pc, a, pl, kc)) : v;
       }
     };
-    team_fft_ex<NY, false, false, true, C::LPV, C::CTA, (BAND ? center_band_mask<NY>() : 0u)>(s, tw, lane, team,
-                                                                                              load1, store1);
+    team_fft_ex<NY, false, false, true, C::LPV, C::CTA>(s, tw, lane, team, load1, store1);
     team_barrier<C::LPV, C::CTA>(team);
     auto load2 = [&](int n) -> float2 { return s[pad_idx(n)]; };
     auto store2 = [&](int k, float2 v, int) { s[pad_idx(k)] = cscale(v, scale); };
@@ -510,14 +522,13 @@ __global__ void __launch_bounds__(RowCfg<NX>::THREADS, RowCfg<NX>::MINB) k_prop_
   }
 }
 
-// the band variants are compiled for lengths of at least 256 whose first
-// radix divides by 4; the data band [pad, pad + n) must lie in [N / 4, 3 N / 4)
-template <int N>
-constexpr bool band_compiled() {
-  return N >= 256 && center_band_mask<N>() != 0u;
-}
-inline bool in_center_band(int N, int pad, int n) { return 4 * pad >= N && 4 * (pad + n) <= 3 * N; }
-
+// the passes on pairs of rows / columns (prop2d_pair.cuh), for lengths with a pair plan
+cx_status dispatch_rows_fwd_pair(int n, const float2* u, float2* T, const Prop2DArgs& a, cudaStream_t st);
+cx_status dispatch_rows_inv_pair(int n, const float2* T2, float2* out, const Prop2DArgs& a, cudaStream_t st);
+cx_status dispatch_cols_pair_eval(int n, const float2* T, float2* T2, const Prop2DArgs& a, cudaStream_t st);
+cx_status dispatch_cols_pair_table(int n, const float2* T, float2* T2, const Prop2DArgs& a, cudaStream_t st);
+cx_status dispatch_cols_pair_eval_odd(int n, const float2* T, float2* T2, const Prop2DArgs& a, cudaStream_t st);
+cx_status dispatch_cols_pair_table_odd(int n, const float2* T, float2* T2, const Prop2DArgs& a, cudaStream_t st);
 // dispatchers (defined in prop2d_rows.cu / prop2d_cols.cu)
 cx_status dispatch_rows_fwd(int n, const float2* u, float2* T, const Prop2DArgs& a, cudaStream_t st);
 cx_status dispatch_cols(int n, const float2* T, float2* T2, const Prop2DArgs& a, cudaStream_t st);

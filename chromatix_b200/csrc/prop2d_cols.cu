@@ -1,4 +1,5 @@
 // Column pass of the Fourier-multiplier propagation (see prop2d.cuh).
+#include "pair_fft.cuh"
 #include "prop2d.cuh"
 
 namespace cx {
@@ -6,18 +7,12 @@ namespace cx {
 template <int NY>
 static cx_status launch_cols(const float2* T, float2* T2, const Prop2DArgs& a, cudaStream_t st) {
   using C = ColCfg<NY>;
-  auto k = k_prop_cols<NY, false>;
+  auto k = k_prop_cols<NY>;
   size_t smem = C::SMEM;
-  const bool band = band_compiled<NY>() && in_center_band(NY, a.pad_y, a.ny);
-  if constexpr (band_compiled<NY>()) {
-    if (band) k = k_prop_cols<NY, true>;
-  }
-  if constexpr (PropColHt<NY>::FITS) {
-    // a propagator table (prop_col mode 4) and no band pruning: stage H with the tile
-    if (!band && a.kernel == CX_KERNEL_EXPLICIT && a.na_f2 < 0.0 && a.H) {
-      k = k_prop_cols<NY, false, true>;
-      smem = PropColHt<NY>::SMEM;
-    }
+  // a propagator table (prop_col mode 4): stage H with the tile
+  if (a.kernel == CX_KERNEL_EXPLICIT && a.na_f2 < 0.0 && a.H) {
+    k = k_prop_cols<NY, true>;
+    smem = PropColHt<NY>::SMEM;
   }
   CX_CUDA_TRY(set_smem(k, smem));
   const long items = (long)((a.px + C::V - 1) / C::V) * a.n_out_planes;
@@ -28,11 +23,18 @@ static cx_status launch_cols(const float2* T, float2* T2, const Prop2DArgs& a, c
 }
 
 cx_status dispatch_cols(int n, const float2* T, float2* T2, const Prop2DArgs& a, cudaStream_t st) {
+  if (pair_length(n)) {
+    const bool table = a.kernel == CX_KERNEL_EXPLICIT;
+    // 16-byte accesses to a column pair
+    const bool vec = a.px % 2 == 0 && ((reinterpret_cast<size_t>(T) | reinterpret_cast<size_t>(T2)) & 15) == 0;
+    if (vec) return table ? dispatch_cols_pair_table(n, T, T2, a, st) : dispatch_cols_pair_eval(n, T, T2, a, st);
+    return table ? dispatch_cols_pair_table_odd(n, T, T2, a, st) : dispatch_cols_pair_eval_odd(n, T, T2, a, st);
+  }
   switch (n) {
 #define CX_CASE_(N) \
   case N:           \
     return launch_cols<N>(T, T2, a, st);
-    CX_FOR_EACH_PROP_SIZE(CX_CASE_)
+    CX_FOR_EACH_SHORT_SIZE(CX_CASE_)
 #undef CX_CASE_
   }
   set_error("FFT length %d is not supported", n);

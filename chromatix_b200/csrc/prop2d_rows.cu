@@ -1,4 +1,5 @@
 // Row passes of the Fourier-multiplier propagation (see prop2d.cuh).
+#include "pair_fft.cuh"
 #include "prop2d.cuh"
 
 namespace cx {
@@ -6,10 +7,7 @@ namespace cx {
 template <int NX>
 static cx_status launch_rows_fwd(const float2* u, float2* T, const Prop2DArgs& a, cudaStream_t st) {
   using C = RowCfg<NX>;
-  auto k = k_prop_rows_fwd<NX, false>;
-  if constexpr (band_compiled<NX>()) {
-    if (in_center_band(NX, a.pad_x, a.nx)) k = k_prop_rows_fwd<NX, true>;
-  }
+  auto k = k_prop_rows_fwd<NX>;
   CX_CUDA_TRY(set_smem(k, C::SMEM));
   const long items = ((long)a.n_in_planes * a.ny + C::TEAMS - 1) / C::TEAMS;
   const int grid = persistent_grid(k, C::THREADS, C::SMEM, items);
@@ -31,11 +29,12 @@ static cx_status launch_rows_inv(const float2* T2, float2* out, const Prop2DArgs
 }
 
 cx_status dispatch_rows_fwd(int n, const float2* u, float2* T, const Prop2DArgs& a, cudaStream_t st) {
+  if (pair_length(n)) return dispatch_rows_fwd_pair(n, u, T, a, st);
   switch (n) {
 #define CX_CASE_(N) \
   case N:           \
     return launch_rows_fwd<N>(u, T, a, st);
-    CX_FOR_EACH_PROP_SIZE(CX_CASE_)
+    CX_FOR_EACH_SHORT_SIZE(CX_CASE_)
 #undef CX_CASE_
   }
   set_error("FFT length %d is not supported", n);
@@ -43,11 +42,12 @@ cx_status dispatch_rows_fwd(int n, const float2* u, float2* T, const Prop2DArgs&
 }
 
 cx_status dispatch_rows_inv(int n, const float2* T2, float2* out, const Prop2DArgs& a, cudaStream_t st) {
+  if (pair_length(n)) return dispatch_rows_inv_pair(n, T2, out, a, st);
   switch (n) {
 #define CX_CASE_(N) \
   case N:           \
     return launch_rows_inv<N>(T2, out, a, st);
-    CX_FOR_EACH_PROP_SIZE(CX_CASE_)
+    CX_FOR_EACH_SHORT_SIZE(CX_CASE_)
 #undef CX_CASE_
   }
   set_error("FFT length %d is not supported", n);

@@ -1,0 +1,100 @@
+"""GPU: the propagation passes on pairs of rows and columns, at every length
+with a plan, rows of odd length, odd numbers of rows, and each way the
+propagator is applied.
+
+Tolerance: an FP32 transform of length N rounds with a relative L2 error of
+about 0.5 eps sqrt(log2 N) <= 1.1e-7, four of them 2.2e-7 added in squares; the
+propagator's hardware sin / cos adds at most 4e-7 (absolute, |H| <= 1).  The
+bar is twice their sum, 1.3e-6.
+"""
+
+import numpy as np
+import pytest
+
+from oracle import chromatix_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+BAR = 1.3e-6
+LENGTHS = [128, 160, 192, 224, 256, 320, 384, 448, 512, 640, 768, 896, 1024, 1280, 1536, 1792, 2048, 2560, 3072, 3584,
+           4096, 8192]
+
+
+def to_cuda(a):
+    import torch
+
+    return torch.as_tensor(a, device="cuda")
+
+
+def _field(u, dx=0.3, lam=0.532):
+    from chromatix_b200.core.field import ChromaticScalarField, ScalarField
+    from chromatix_b200.core.spectrum import Spectrum
+
+    spec = Spectrum.build(lam)
+    cls = ChromaticScalarField if spec.size > 1 else ScalarField
+    return cls(to_cuda(u), dx, 0.0, spec)
+
+
+def _crand(rng, shape):
+    return (rng.standard_normal(shape) + 1j * rng.standard_normal(shape)).astype(np.complex64)
+
+
+@pytest.mark.parametrize("n", LENGTHS)
+def test_table_propagator_every_length(n):
+    import chromatix_b200.functional as cf
+
+    rng = np.random.default_rng(n)
+    # columns of length n with a ragged last tile (10 columns), with odd rows (5), and rows of length n
+    for shape in ((n, 10), (n, 5), (6, n)):
+        u = _crand(rng, (3,) + shape)
+        H = _crand(rng, shape)
+        out = cf.kernel_propagate(_field(u), to_cuda(H)).u.cpu().numpy()
+        ref = np.fft.ifft2(np.fft.fft2(u.astype(np.complex128)) * H)
+        assert O.rel_l2(out, ref) < BAR, shape
+
+
+@pytest.mark.parametrize("n", LENGTHS)
+def test_evaluated_propagator_every_length(n):
+    import chromatix_b200.functional as cf
+
+    rng = np.random.default_rng(n + 1)
+    z = [40.0, 40.0, -15.0]  # a plane with its predecessor's propagator, then another
+    # padded on both sides, an odd number of data rows never divides into pairs
+    for ny, nx, pad in ((n - 2 * (n // 5), 4, (n // 5, 1)), (n // 2, 6, (n // 4, 0))):
+        u = _crand(rng, (3, ny, nx))
+        f = _field(u)
+        for kw in (dict(mode="same"), dict(mode="full", shift_yx=(1.5, -0.7)), dict(mode="full", kykx=(0.2, 0.1))):
+            out = cf.asm_propagate(f, np.array(z), 1.33, pad, **kw).u.cpu().numpy()
+            for b in range(3):
+                ref = O.asm_propagate(O.field_build(u[b], 0.3, 0.532), z[b], 1.33, pad, **kw).u
+                assert O.rel_l2(out[b], np.asarray(ref).reshape(out[b].shape)) < BAR, (ny, kw, b)
+
+
+@pytest.mark.parametrize("ny,nx,pad", [(101, 131, (21, 29)), (77, 96, (26, 16))])
+def test_odd_rows_and_wavelengths(ny, nx, pad):
+    """Odd numbers of rows with two wavelengths innermost, forward and gradient."""
+    import torch
+
+    import chromatix_b200.functional as cf
+
+    # padded to lengths with a plan (odd fields: odd padded lengths go another way, so pad unevenly sized fields)
+    ny, nx = ny + ny % 2, nx + nx % 2
+    rng = np.random.default_rng(5)
+    u = _crand(rng, (2, ny, nx, 2))
+    lam = np.array([0.45, 0.6])
+    f = _field(u, lam=lam)
+    f.u.requires_grad_(True)
+    py = min(n for n in LENGTHS if n >= ny + pad[0])
+    px = min(n for n in LENGTHS if n >= nx + pad[1])
+    pads = ((py - ny) // 2, (px - nx) // 2)
+    out = cf.transfer_propagate(f, 30.0, 1.33, pads, mode="same")
+    g = _crand(rng, out.u.shape)
+    (gu,) = torch.autograd.grad(out.u, f.u, to_cuda(g))
+    for w in range(2):
+        fy, fx = np.fft.fftfreq(py, 0.3), np.fft.fftfreq(px, 0.3)
+        H = np.exp(-1j * np.pi * lam[w] * 30.0 / 1.33 * (fy[:, None] ** 2 + fx[None, :] ** 2))
+        for src, h, dst in ((u, H, out.u.detach().cpu().numpy()), (g, H.conj(), gu.cpu().numpy())):
+            for b in range(2):
+                v = np.pad(src[b, :, :, w].astype(np.complex128), [(p, p) for p in pads])
+                ref = np.fft.ifft2(np.fft.fft2(v) * h)[pads[0]:pads[0] + ny, pads[1]:pads[1] + nx]
+                assert O.rel_l2(dst[b, :, :, w], ref) < BAR
