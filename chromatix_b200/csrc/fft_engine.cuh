@@ -516,17 +516,6 @@ __device__ __forceinline__ void team_fft(float2* s, const float2* tw, int lane, 
   Stage<N, LPV, INV, 0, 1, CTA, ZM>::run(s, tw, lane, team, load, store);
 }
 
-// Zero mask for team_fft when the input vector is nonzero only on
-// [0, h) and [N - h, N) with h <= Q N / R_0 (a centred support after an
-// ifftshift): first-stage inputs r in [Q, R_0 - Q) are zero.
-template <int N, int Q>
-__host__ __device__ constexpr unsigned edge_zero_mask() {
-  constexpr int R0 = Plan<N>::P.r[0];
-  unsigned m = 0u;
-  for (int r = Q; r < R0 - Q; ++r) m |= 1u << r;
-  return m;
-}
-
 // First-stage zero mask for an input that is nonzero only on [0, N / 2)
 // (zero padding to twice the length): with an even first radix R_0 the
 // inputs r >= R_0 / 2 of every first-stage butterfly (indices

@@ -438,6 +438,20 @@ struct PairFFT {
     });
   }
 
+  // last stage with the outputs left in the buffer: frequency k = b + r N / RL at last_ptr(b) + r VP
+  template <bool INV>
+  __device__ __forceinline__ static void last_in_place(float4* s, int t) {
+    each<N / RL>(t, [&](int b) {
+      float4* p = last_ptr(s, b);
+      c2 v[RL];
+#pragma unroll
+      for (int r = 0; r < RL; ++r) v[r] = sload(p + r * VP);
+      PDFT<RL, INV>::run(v);
+#pragma unroll
+      for (int r = 0; r < RL; ++r) sstore(p + r * VP, v[r]);
+    });
+  }
+
   // centre of a round trip over butterflies [b0, b1): last stage, v <- f(b, r, v) at frequency b + r N / RL,
   // first stage back, in place.  Rolled: the body is emitted once.
   template <bool INV, class G>
@@ -480,20 +494,11 @@ struct PairFFT {
   }
 };
 
-// first-stage inputs that are zero when the vector lives on the ends [0, Q M)
-// and [N - Q M, N) (a centred support after an ifftshift)
-template <int N, int Q>
-constexpr unsigned pair_edge_mask() {
-  unsigned m = 0u;
-  for (int r = Q; r < PairPlan<N>::R1 - Q; ++r) m |= 1u << r;
-  return m;
-}
-
 // Row kernels on pairs of rows: one buffer per pair, TEAMS pairs per CTA.
 // Pairs of whole warps synchronise on a named barrier of their own; pairs that
 // do not tile warps run in lockstep on the CTA's barrier (every team of the
 // CTA then runs the same number of transforms).
-template <int N, int TARGET = 128>
+template <int N, int TARGET = 128, int LANES = 512>
 struct PairRows {
   using F = PairFFT<N, 1>;
   static constexpr int L = F::L;
@@ -509,8 +514,9 @@ struct PairRows {
   static constexpr int THREADS = TEAMS * L;
   static constexpr int TWB = (F::TW * (int)sizeof(float2) + 15) & ~15;
   static constexpr size_t SMEM = TWB + sizeof(float4) * (size_t)TEAMS * F::ELEMS;
-  // 128 registers hold a radix-16 stage of a pair (64 for the values, the rest addresses and twiddles)
-  static constexpr int MINB = 512 / THREADS > 0 ? 512 / THREADS : 1;
+  // LANES resident lanes per SM set the register budget: at 512, 128 registers hold a radix-16 stage of a pair (64
+  // for the values, the rest addresses and twiddles); at 640, 96 just do
+  static constexpr int MINB = LANES / THREADS > 0 ? LANES / THREADS : 1;
   __device__ __forceinline__ static void sync(int team) {
     if constexpr (OWN) {
       asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(L) : "memory");

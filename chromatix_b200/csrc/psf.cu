@@ -42,12 +42,12 @@ __global__ void k_psf_count(PsfArgs a, unsigned long long* counts, int* srange) 
 }
 
 // ---------------------------------------------------------------------------
-// accurate-mode source tables (PsfArgs::M, PsfArgs::CX), FP64 phases
+// accurate-mode source tables (PsfArgs::M, PsfArgs::CX, PsfArgs::CY), FP64 phases
 // ---------------------------------------------------------------------------
 __global__ void k_psf_tables(PsfArgs a) {
-  const long ncx = (long)a.nz * a.csum;
+  const long ncx = (long)a.nz * a.csum, ncy = (long)a.nz * a.rowsum;
   const double PI = 3.141592653589793238462643383279502884;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < a.msum + ncx; i += (long)gridDim.x * blockDim.x) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < a.msum + ncx + ncy; i += (long)gridDim.x * blockDim.x) {
     if (i < a.msum) {
       int w = 0;
       while (w + 1 < a.W && i >= a.mprefix[w + 1]) ++w;
@@ -60,6 +60,16 @@ __global__ void k_psf_tables(PsfArgs a) {
         if (a.has_phase) v = cmul(v, expi_precise((double)a.phase[(size_t)y * a.nx + x] * p.mod));
       }
       a.M[i] = v;
+    } else if (i >= a.msum + ncx) {
+      const long j = i - a.msum - ncx;
+      const int iz = (int)(j / a.rowsum), loc = (int)(j % a.rowsum);
+      int w = 0;
+      while (w + 1 < a.W && loc >= a.prefix[w + 1]) ++w;
+      const PsfWv& p = a.wv[w];
+      const int y = a.ylo[w] + (loc - a.prefix[w]);
+      const double gyo = p.dy * ((double)y - (double)a.ny * 0.5) - a.offy;
+      const double qz = -PI * (a.z[iz] / a.f_obj) / p.L2;
+      a.CY[j] = expi_precise(qz * gyo * gyo);
     } else {
       const long j = i - a.msum;
       const int iz = (int)(j / a.csum), loc = (int)(j % a.csum);
@@ -157,15 +167,17 @@ static void psf_cols_box(const cx_psf_desc* d, const cx_psf_spectrum* spec, int 
   *ncols = (int)(hi - lo + 1);
 }
 
-// Row spectra of one z-chunk are written by pass A and read back by pass B;
-// the chunk is sized to stay L2-resident in between (CX_PSF_L2_MB, default
-// 64 MiB of the 126 MB L2).
+// Row spectra of one z-chunk are written by pass A and read back by pass B.
+// 512 MiB (CX_PSF_CHUNK_MB): chunks that stay in the 126 MB L2 launch each
+// pass on three planes of a 3 x 1280^2 stack, and the launches' ramps and last
+// waves cost more than the spectra's way through HBM (64 planes, chunk in MiB:
+// 44 2023 us, 64 2103, 132 1930, 264 1753, 600 1702, all planes at once 1670).
 static size_t psf_chunk_budget() {
   static size_t cached = 0;
   if (!cached) {
-    const char* e = getenv("CX_PSF_L2_MB");
-    const long mb = e ? atol(e) : 64;
-    cached = (size_t)(mb > 0 ? mb : 64) << 20;
+    const char* e = getenv("CX_PSF_CHUNK_MB");
+    const long mb = e ? atol(e) : 512;
+    cached = (size_t)(mb > 0 ? mb : 512) << 20;
   }
   return cached;
 }
@@ -248,17 +260,23 @@ static PsfArgs psf_make_args(const cx_psf_desc* d, const cx_psf_spectrum* spec, 
 
 // workspace: 256 bytes of pupil counters, then one chunk of row spectra
 // (sized for the worst case rowsum = n_wv * ny, independent of the spectrum)
+static int psf_ld(const cx_psf_desc* d) { return d->nx + d->nx % 2; }
 static size_t psf_t_bytes(const cx_psf_desc* d) {
-  const size_t worst_z = (size_t)d->n_wv * d->ny * d->nx * sizeof(float2);
-  const size_t t = psf_chunk_budget() > worst_z ? psf_chunk_budget() : worst_z;
+  const size_t worst_z = (size_t)d->n_wv * d->ny * psf_ld(d) * sizeof(float2);
+  // at least one plane, at most all of them
+  const size_t need = worst_z * (size_t)d->n_z;
+  size_t t = psf_chunk_budget() > worst_z ? psf_chunk_budget() : worst_z;
+  if (t > need) t = need;
   return (t + 255) & ~(size_t)255;
 }
 static size_t psf_m_bytes(const cx_psf_desc* d) {
   return ((size_t)d->n_wv * d->ny * d->nx * sizeof(float2) + 255) & ~(size_t)255;
 }
+static size_t psf_cx_bytes(const cx_psf_desc* d) {
+  return ((size_t)d->n_z * d->n_wv * d->nx * sizeof(float2) + 255) & ~(size_t)255;
+}
 static size_t psf_ws(const cx_psf_desc* d) {
-  const size_t cx_bytes = ((size_t)d->n_z * d->n_wv * d->nx * sizeof(float2) + 255) & ~(size_t)255;
-  return 256 + psf_t_bytes(d) + psf_m_bytes(d) + cx_bytes;
+  return 256 + psf_t_bytes(d) + psf_m_bytes(d) + psf_cx_bytes(d) + sizeof(float2) * (size_t)d->n_z * d->n_wv * d->ny;
 }
 
 }  // namespace cx
@@ -314,8 +332,10 @@ static cx_status psf_setup(const cx_psf_desc* d, const cx_psf_spectrum* spec, co
   }
   a.M = reinterpret_cast<float2*>(static_cast<char*>(workspace) + 256 + psf_t_bytes(d));
   a.CX = reinterpret_cast<float2*>(static_cast<char*>(workspace) + 256 + psf_t_bytes(d) + psf_m_bytes(d));
+  a.CY = a.CX + psf_cx_bytes(d) / sizeof(float2);
+  a.ldT = psf_ld(d);
   // z planes per chunk: as many compact planes as the row-spectrum region holds
-  const size_t zbytes = sizeof(float2) * (size_t)a.rowsum * a.nx;
+  const size_t zbytes = sizeof(float2) * (size_t)a.rowsum * a.ldT;
   int zc = (int)(psf_t_bytes(d) / zbytes);
   if (zc < 1) zc = 1;
   if (zc > a.nz) zc = a.nz;
@@ -330,7 +350,7 @@ static cx_status psf_prepare(const PsfArgs& a, void* workspace, cudaStream_t st)
                                                          const_cast<int*>(a.srange));
   CX_LAUNCH_CHECK();
   if (a.precision != CX_PREC_REF32) {
-    const long n = a.msum + (long)a.nz * a.csum;
+    const long n = a.msum + (long)a.nz * (a.csum + a.rowsum);
     const int blocks = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
     k_psf_tables<<<blocks, 256, 0, st>>>(a);
     CX_LAUNCH_CHECK();
@@ -370,7 +390,7 @@ extern "C" cx_status cx_psf_plan_info(const cx_psf_desc* d, const cx_psf_spectru
     psf_rows(d, spec, w, &lo, &nr);
     rowsum += nr;
   }
-  const size_t zbytes = sizeof(float2) * (size_t)rowsum * d->nx;
+  const size_t zbytes = sizeof(float2) * (size_t)rowsum * psf_ld(d);
   int zc = (int)(psf_t_bytes(d) / zbytes);
   if (zc < 1) zc = 1;
   if (zc > d->n_z) zc = d->n_z;
@@ -410,19 +430,20 @@ namespace cx {
 constexpr int kPsfHostSlots = 3;
 constexpr int kPsfHostGroups = 8;  // target number of copy groups per stack
 
-// group = z-planes per copy group; first = planes of the first group (one
-// chunk, so that the first copy starts early)
+// group = z-planes per copy group; first = planes of the first group (a third,
+// so that the first copy starts early)
 static cx_status psf_host_plan(const cx_psf_desc* d, const cx_psf_spectrum* spec, int* group, size_t* slot_bytes,
                                int* first = nullptr) {
   int32_t info[4];
   cx_status s = cx_psf_plan_info(d, spec, info);
   if (s != CX_OK) return s;
-  const int zc = info[0], chunks = info[2];
-  const int per_group = (chunks + kPsfHostGroups - 1) / kPsfHostGroups;
-  int g = zc * (per_group > 0 ? per_group : 1);
+  // an eighth of the stack, in whole chunks where it is more than one
+  const int zc = info[0];
+  int g = (d->n_z + kPsfHostGroups - 1) / kPsfHostGroups;
+  if (g > zc) g = (g + zc - 1) / zc * zc;
   if (g > d->n_z) g = d->n_z;
   *group = g;
-  if (first) *first = zc < g ? zc : g;
+  if (first) *first = (g + 2) / 3;
   *slot_bytes = (((size_t)g * d->ny * d->nx * sizeof(float)) + 255) & ~(size_t)255;
   return CX_OK;
 }

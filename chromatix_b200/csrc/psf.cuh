@@ -16,8 +16,8 @@
 // pass B  per (z, V-column tile): for every wavelength FFT along y and add
 //         density * |X|^2 into per-lane registers; store the fftshifted
 //         intensity once.
-// The z axis is processed in chunks so the row spectra of a chunk stay in L2
-// between pass A and pass B.
+// The z axis is processed in chunks, as many planes as fit the row-spectrum
+// workspace.
 #pragma once
 #include "host.cuh"
 
@@ -52,9 +52,12 @@ struct PsfArgs {
   int csum;
   float2* M;
   float2* CX;
+  // CY (nz, rowsum), by stored row: exp(i qz (y dy - off_y)^2) (pair passes)
+  float2* CY;
+  int ldT;  // row pitch of T: nx, rounded up to even
   const double* z;
   const float* phase;
-  float2* T;  // (zc, rowsum, nx): only the rows [ylo_w, ylo_w + nrows_w) of each wavelength
+  float2* T;  // (zc, rowsum, ldT): only the rows [ylo_w, ylo_w + nrows_w) of each wavelength
   const unsigned long long* counts;  // [0, 8): pupil pixel counts per wavelength
   const int* srange;                 // [0, 8): ny - first support row ; [8, 16): last support row + 1
   float* out;
@@ -119,7 +122,7 @@ __device__ __forceinline__ float2 psf_const(const PsfArgs& a, int w, const unsig
 template <int NX>
 using PsfRowCfg = RowCfgX<NX>;
 
-template <int NX, int Q>
+template <int NX>
 __global__ void __launch_bounds__(PsfRowCfg<NX>::THREADS, PsfRowCfg<NX>::MINB) k_psf_rows_tab(PsfArgs a) {
   using C = PsfRowCfg<NX>;
   extern __shared__ float2 sm[];
@@ -147,7 +150,7 @@ __global__ void __launch_bounds__(PsfRowCfg<NX>::THREADS, PsfRowCfg<NX>::MINB) k
     const float2* cxz = a.CX + (size_t)(a.z0 + zl) * a.csum + a.cprefix[w];
     const int xlo = a.xlo[w], nc = live ? a.ncols[w] : 0;
     const float2 cy = expi_precise(qz * gyo * gyo);
-    float2* dst = a.T + ((size_t)zl * a.rowsum + rem) * a.nx;
+    float2* dst = a.T + ((size_t)zl * a.rowsum + rem) * a.ldT;
     auto load = [&](int n) -> float2 {
       const int c = add_mod(n, NX / 2, NX) - xlo;  // ifftshift along x, then the box column
       if ((unsigned)c >= (unsigned)nc) return make_float2(0.f, 0.f);
@@ -156,7 +159,7 @@ __global__ void __launch_bounds__(PsfRowCfg<NX>::THREADS, PsfRowCfg<NX>::MINB) k
     auto store = [&](int k, float2 v, int) {
       if (live) dst[k] = v;
     };
-    team_fft<NX, false, C::LPV, C::CTA, (Q > 0 ? edge_zero_mask<NX, Q>() : 0u)>(s, tw, lane, team, load, store);
+    team_fft<NX, false, C::LPV, C::CTA>(s, tw, lane, team, load, store);
   }
 }
 
@@ -192,7 +195,7 @@ __global__ void __launch_bounds__(RowCfg<NX>::THREADS, RowCfg<NX>::MINB) k_psf_r
     const double gy = p.dy * ((double)y - (double)a.ny * 0.5);
     const double qz = -PI * (z / a.f_obj) / p.L2;
     const double gyo = gy - a.offy;
-    float2* dst = a.T + ((size_t)zl * a.rowsum + rem) * a.nx;
+    float2* dst = a.T + ((size_t)zl * a.rowsum + rem) * a.ldT;
     auto store = [&](int k, float2 v, int) { dst[k] = v; };
     auto load = [&](int n) -> float2 {
       const int x = add_mod(n, NX / 2, NX);  // ifftshift along x
@@ -234,9 +237,7 @@ struct PsfColCfg {
   static constexpr size_t SMEM = ((C::SMEM + 15) & ~(size_t)15) + sizeof(float) * (size_t)C::V * ACC;
 };
 
-// Q > 0: every wavelength's pupil rows map to FFT rows within Q N/R_0 of the
-// ends (checked on the host), so the first stage skips the zero inputs
-template <int NY, int Q>
+template <int NY>
 __global__ void __launch_bounds__(ColCfg<NY>::THREADS, ColCfg<NY>::MINB) k_psf_cols(PsfArgs a) {
   using C = ColCfg<NY>;
   constexpr int V = C::V, LEN = C::LEN, ACC = PsfColCfg<NY>::ACC;
@@ -256,12 +257,12 @@ __global__ void __launch_bounds__(ColCfg<NY>::THREADS, ColCfg<NY>::MINB) k_psf_c
     for (int w = 0; w < a.W; ++w) {
       const PsfWv& p = a.wv[w];
       const float dens = (float)p.dens;
-      const float2* src = a.T + ((size_t)zl * a.rowsum + a.prefix[w]) * a.nx;
+      const float2* src = a.T + ((size_t)zl * a.rowsum + a.prefix[w]) * a.ldT;
       const int ylo = a.ylo[w];
       const int slo = support_lo(a, w), shi = support_hi(a, w);
       __syncthreads();
       // field rows [slo, shi) feed FFT rows (y - ny/2) mod ny (ifftshift)
-      load_col_tile<V, LEN>(tile, src - (size_t)ylo * a.nx, a.nx, x0, a.nx, slo, shi,
+      load_col_tile<V, LEN>(tile, src - (size_t)ylo * a.ldT, a.ldT, x0, a.nx, slo, shi,
                             [&](int y) { return add_mod(y, NY - NY / 2, NY); });
       __syncthreads();
       // FFT row n holds field row (n + NY/2) mod NY; the support [slo, shi)
@@ -275,7 +276,7 @@ __global__ void __launch_bounds__(ColCfg<NY>::THREADS, ColCfg<NY>::MINB) k_psf_c
         const float e = dens * cabs2(v);
         acc[k] = (w == 0) ? e : acc[k] + e;
       };
-      team_fft<NY, false, C::LPV, C::CTA, (Q > 0 ? edge_zero_mask<NY, Q>() : 0u)>(s, tw, lane, team, load, store);
+      team_fft<NY, false, C::LPV, C::CTA>(s, tw, lane, team, load, store);
     }
     __syncthreads();
     float* outz = a.out + (size_t)(a.z0 + zl) * a.ny * a.nx;
@@ -292,28 +293,9 @@ __global__ void __launch_bounds__(ColCfg<NY>::THREADS, ColCfg<NY>::MINB) k_psf_c
 // accurate-mode source tables M and CX (see PsfArgs), after the count pass
 __global__ void k_psf_tables(PsfArgs a);
 
-// The pupil boxes of every wavelength (rows [ylo, ylo + nrows) or columns
-// [xlo, xlo + ncols) of a length-n axis) map, after the ifftshift, to FFT
-// indices within q n / r0 of both ends
-inline bool psf_edges_within(const PsfArgs& a, bool rows, int n, int r0, int q) {
-  const long lim = (long)q * (n / r0);
-  for (int w = 0; w < a.W; ++w) {
-    const long lo = rows ? a.ylo[w] : a.xlo[w];
-    const long hi = lo + (rows ? a.nrows[w] : a.ncols[w]);  // exclusive
-    if (hi - n / 2 > lim || n / 2 - lo > lim) return false;
-  }
-  return true;
-}
-
-// the narrowest first-stage band (in units of N / R_0 from each end) that
-// holds every wavelength's pupil box: 3, 4 or 6, else 0 (dense)
-inline int psf_edge_q(const PsfArgs& a, bool rows, int n, int r0) {
-  if (r0 < 16) return 0;
-  for (int q : {3, 4, 6})
-    if (psf_edges_within(a, rows, n, r0, q)) return q;
-  return 0;
-}
-
+// the passes on pairs of rows / columns (psf_pair.cuh), for lengths with a pair plan
+cx_status psf_dispatch_rows_pair(int n, const PsfArgs& a, cudaStream_t st);
+cx_status psf_dispatch_cols_pair(int n, const PsfArgs& a, cudaStream_t st);
 cx_status psf_dispatch_rows(int n, const PsfArgs& a, cudaStream_t st);
 cx_status psf_dispatch_cols(int n, const PsfArgs& a, cudaStream_t st);
 // CX_PREC_SPLIT16 column pass on the tensor cores (psf_tc.cu)

@@ -98,3 +98,25 @@ def test_odd_rows_and_wavelengths(ny, nx, pad):
                 v = np.pad(src[b, :, :, w].astype(np.complex128), [(p, p) for p in pads])
                 ref = np.fft.ifft2(np.fft.fft2(v) * h)[pads[0]:pads[0] + ny, pads[1]:pads[1] + nx]
                 assert O.rel_l2(dst[b, :, :, w], ref) < BAR
+
+
+@pytest.mark.parametrize("ny,nx,wv", [(128, 128, 3), (160, 10, 1), (224, 5, 2), (320, 448, 1), (768, 256, 2),
+                                      (1280, 192, 3), (2048, 128, 1), (192, 4096, 1), (4096, 128, 2)])
+def test_psf_stack(ny, nx, wv):
+    """The fused PSF: stored row spectra of odd and even pitch, row boxes of odd height, an offset source, one and
+    several wavelengths (tolerance of the intensity: twice the field's, and the source's sin / cos are FP64)."""
+    import chromatix_b200.functional as cf
+
+    rng = np.random.default_rng(ny + nx)
+    wl = np.array([0.532, 0.45, 0.63][:wv])
+    dx = 8000.0 * 0.532 / (1.33 * 0.35 * min(ny, nx)) * 0.01 * (wl / 0.532)
+    z = np.array([-3.0, 0.5, 4.0])
+    spec = (wl, np.arange(1.0, wv + 1)) if wv > 1 else float(wl[0])
+    phase = rng.uniform(0, 2 * np.pi, (ny, nx)).astype(np.float32)
+    NA = 0.8 * 1.33 * min(ny, nx) / 2 * float(dx.min()) / 8000.0  # a pupil of 0.8 of the shorter side
+    args = ((ny, nx), dx if wv > 1 else float(dx[0]), spec, z, 8000.0, 1.33, NA)
+    off = (0.3 * float(dx[0]), -0.2 * float(dx[0]))
+    f = cf.objective_point_source(*args, offset=off, device="cuda")
+    out = cf.ff_lens(cf.phase_change(f, to_cuda(phase)), 200000.0, 1.33).intensity.cpu().numpy()
+    ref = O.ff_lens(O.phase_change(O.objective_point_source(*args, offset=off), phase), 200000.0, 1.33).intensity
+    assert O.rel_l2(out, np.asarray(ref).reshape(out.shape)) < 2 * BAR
