@@ -1,6 +1,7 @@
 // C API of the plane-wise Fourier convolution with the sensor's plane sum
 // (kernels in conv.cuh).
 #include "conv.cuh"
+#include "conv_pair.cuh"
 
 namespace cx {
 
@@ -64,7 +65,9 @@ static cx_status conv_plan(const cx_conv_desc* d, ConvArgs* a, int* zc, size_t* 
   a->c0y = (d->kh - 1) / 2;
   a->c0x = (d->kw - 1) / 2;
   a->scale = (float)(2.0 / ((double)a->P * (double)a->Q));
-  const size_t plane_t = sizeof(float2) * 2 * (size_t)a->HB * a->NT * vt;
+  a->ldY = a->HB + a->HB % 2;
+  const size_t plane_t = conv_on_pairs(a->M, a->P) ? sizeof(float4) * (size_t)a->NC * a->ldY
+                                                   : sizeof(float2) * 2 * (size_t)a->HB * a->NT * vt;
   int c = (int)(kConvChunkBytes / plane_t);
   if (c < 1) c = 1;
   if (c > d->n_planes) c = d->n_planes;
@@ -117,6 +120,7 @@ extern "C" cx_status cx_conv2d_same(const cx_conv_desc* d, const float* sample, 
   const size_t st_bytes = sizeof(float2) * (size_t)a.NC * a.P;
   const size_t img = (size_t)d->h * d->w;
   // reduce: one accumulated spectrum for all planes; otherwise one per plane
+  const bool pairs = conv_on_pairs(a.M, a.P);
   const int groups = d->reduce ? 1 : d->n_planes;
   for (int g = 0; g < groups; ++g) {
     const int p_lo = d->reduce ? 0 : g, p_hi = d->reduce ? d->n_planes : g + 1;
@@ -124,8 +128,13 @@ extern "C" cx_status cx_conv2d_same(const cx_conv_desc* d, const float* sample, 
     for (int z0 = p_lo; z0 < p_hi; z0 += zc) {
       a.z0 = z0;
       a.zc = (p_hi - z0) < zc ? (p_hi - z0) : zc;
-      if ((s = conv_dispatch_rows(a.M, a, st)) != CX_OK) return s;
-      if ((s = conv_dispatch_cols(a.P, a, st)) != CX_OK) return s;
+      if (pairs) {
+        if ((s = conv_dispatch_rows_pair(a.M, a, st)) != CX_OK) return s;
+        if ((s = conv_dispatch_cols_pair(a.P, a, st)) != CX_OK) return s;
+      } else {
+        if ((s = conv_dispatch_rows(a.M, a, st)) != CX_OK) return s;
+        if ((s = conv_dispatch_cols(a.P, a, st)) != CX_OK) return s;
+      }
     }
     a.out = out + (size_t)g * img;
     if ((s = conv_dispatch_fin_cols(a.P, a, st)) != CX_OK) return s;

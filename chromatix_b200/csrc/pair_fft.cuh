@@ -75,6 +75,28 @@ __device__ __forceinline__ c2 sload(const float4* s) {
 }
 __device__ __forceinline__ void sstore(float4* s, c2 a) { *s = make_float4(a.re.x, a.re.y, a.im.x, a.im.y); }
 
+// Predicated global loads, zero where !ok.  As one instruction each (not a
+// branch around a load and its use) all loads of a stage are issued before the
+// first is waited for.  volatile: they stay behind barriers and grid waits.
+__device__ __forceinline__ float4 ld4z(const void* p, bool ok) {
+  float4 v;
+  asm volatile(
+      "{\n .reg .pred q;\n setp.ne.u32 q, %5, 0;\n mov.f32 %0, 0f00000000;\n mov.f32 %1, 0f00000000;\n"
+      " mov.f32 %2, 0f00000000;\n mov.f32 %3, 0f00000000;\n @q ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];\n}"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "l"(p), "r"((unsigned)ok));
+  return v;
+}
+__device__ __forceinline__ float2 ld2z(const void* p, bool ok) {
+  float2 v;
+  asm volatile(
+      "{\n .reg .pred q;\n setp.ne.u32 q, %3, 0;\n mov.f32 %0, 0f00000000;\n mov.f32 %1, 0f00000000;\n"
+      " @q ld.global.v2.f32 {%0, %1}, [%2];\n}"
+      : "=f"(v.x), "=f"(v.y)
+      : "l"(p), "r"((unsigned)ok));
+  return v;
+}
+
 // ---------------------------------------------------------------------------
 // small DFTs of c2 (natural order in and out)
 // ---------------------------------------------------------------------------
@@ -245,6 +267,10 @@ struct PDFT<14, INV> : PDFTGood<2, 7, INV> {};
 // lanes: the row passes of 64 1024^2 fields went from 78 to 81 and from 174 to
 // 176 us.  With w and w^4 only, the error against FP64 was a tenth larger.)
 __host__ __device__ constexpr int ptw_powers(int R) { return R > 8 ? 4 : (R > 4 ? 3 : (R > 2 ? 2 : 1)); }
+// (cmul with the contraction written out: every kernel forms the same bits)
+__device__ __forceinline__ float2 cmul_rn(float2 a, float2 b) {
+  return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
 template <int R, bool CONJ, int BLOCK>
 __device__ __forceinline__ void ptwiddle(c2* v, const float2* tw) {
   const float2 w1 = tw[0];
@@ -253,7 +279,7 @@ __device__ __forceinline__ void ptwiddle(c2* v, const float2* tw) {
     const float2 w2 = tw[BLOCK];
     v[2] = pmulw<CONJ>(v[2], w2);
     if constexpr (R > 3) {
-      const float2 w3 = cmul(w2, w1);
+      const float2 w3 = cmul_rn(w2, w1);
       v[3] = pmulw<CONJ>(v[3], w3);
       if constexpr (R > 4) {
         const float2 w4 = tw[2 * BLOCK];
@@ -261,11 +287,11 @@ __device__ __forceinline__ void ptwiddle(c2* v, const float2* tw) {
 #pragma unroll
         for (int q = 1; 4 * q < R; ++q) {
           if (q == 2) wq = tw[3 * BLOCK];
-          if (q == 3) wq = cmul(wq, w4);
+          if (q == 3) wq = cmul_rn(wq, w4);
           v[4 * q] = pmulw<CONJ>(v[4 * q], wq);
-          if (4 * q + 1 < R) v[4 * q + 1] = pmulw<CONJ>(v[4 * q + 1], cmul(wq, w1));
-          if (4 * q + 2 < R) v[4 * q + 2] = pmulw<CONJ>(v[4 * q + 2], cmul(wq, w2));
-          if (4 * q + 3 < R) v[4 * q + 3] = pmulw<CONJ>(v[4 * q + 3], cmul(wq, w3));
+          if (4 * q + 1 < R) v[4 * q + 1] = pmulw<CONJ>(v[4 * q + 1], cmul_rn(wq, w1));
+          if (4 * q + 2 < R) v[4 * q + 2] = pmulw<CONJ>(v[4 * q + 2], cmul_rn(wq, w2));
+          if (4 * q + 3 < R) v[4 * q + 3] = pmulw<CONJ>(v[4 * q + 3], cmul_rn(wq, w3));
         }
       }
     }
@@ -291,17 +317,35 @@ __device__ __forceinline__ void ptwiddle(c2* v, const float2* tw) {
   X(3072, 192, 16, 16, 12, 1) X(3584, 224, 16, 16, 14, 1) X(4096, 256, 16, 16, 16, 1)
 #define CX_PAIR_PLANS(X) CX_PAIR_PLANS_4096(X) X(8192, 512, 16, 8, 8, 8)
 
+template <int N, bool LONE = false>
+struct PairPlan : PairPlan<N, false> {};
 template <int N>
-struct PairPlan {
+struct PairPlan<N, false> {
   static constexpr int L = 0, R1 = 0, R2 = 0, R3 = 0, R4 = 0;
 };
 #define CX_PAIR_PLAN_(N_, L_, A_, B_, C_, D_)                                          \
   template <>                                                                          \
-  struct PairPlan<N_> {                                                                \
+  struct PairPlan<N_, false> {                                                         \
     static constexpr int L = L_, R1 = A_, R2 = B_, R3 = C_, R4 = D_;                   \
     static_assert(A_ * B_ * C_ * D_ == N_ && N_ / A_ % L_ == 0 && N_ / A_ % 2 == 0, ""); \
   };
 CX_PAIR_PLANS(CX_PAIR_PLAN_)
+#undef CX_PAIR_PLAN_
+
+// LONE: plans for passes over one plane, where a pass is a single wave and
+// its time the length of one lane's work: 8 points per lane where the plans
+// above have 16, at the price of a fourth stage from 1024 up.
+#define CX_PAIR_LONE_PLANS(X)                                                                           \
+  X(640, 80, 8, 8, 10, 1) X(768, 96, 8, 8, 12, 1) X(896, 112, 8, 8, 14, 1) X(1024, 128, 8, 8, 4, 4)     \
+  X(1280, 160, 8, 8, 5, 4) X(1536, 192, 8, 8, 6, 4) X(1792, 224, 8, 8, 7, 4) X(2048, 256, 8, 8, 8, 4)   \
+  X(2560, 320, 8, 8, 10, 4) X(3072, 384, 8, 8, 12, 4) X(3584, 448, 8, 8, 14, 4) X(4096, 512, 8, 8, 16, 4)
+#define CX_PAIR_PLAN_(N_, L_, A_, B_, C_, D_)                                          \
+  template <>                                                                          \
+  struct PairPlan<N_, true> {                                                          \
+    static constexpr int L = L_, R1 = A_, R2 = B_, R3 = C_, R4 = D_;                   \
+    static_assert(A_ * B_ * C_ * D_ == N_ && N_ / A_ % L_ == 0 && N_ / A_ % 2 == 0, ""); \
+  };
+CX_PAIR_LONE_PLANS(CX_PAIR_PLAN_)
 #undef CX_PAIR_PLAN_
 
 template <int N>
@@ -322,9 +366,9 @@ inline bool pair_length(int n) {
 // One transform length on VP interleaved pairs per buffer.  `t` is the lane
 // inside the pair (0 .. L-1); `s` points at the pair's element 0 (its index c
 // is already added); `tw` at the twiddle tables in shared memory (TW float2).
-template <int N, int VP = 1>
+template <int N, int VP = 1, bool LONE = false>
 struct PairFFT {
-  using P = PairPlan<N>;
+  using P = PairPlan<N, LONE>;
   static constexpr int L = P::L, R1 = P::R1, R2 = P::R2, R3 = P::R3, R4 = P::R4;
   static constexpr int S = R3 == 1 ? 2 : (R4 == 1 ? 3 : 4);
   static constexpr int M = N / R1, M2 = M / R2, M3 = M2 / R3;  // block lengths
@@ -421,12 +465,9 @@ struct PairFFT {
     }
   }
 
-  // transform: out(k, v) for every k (unnormalised); the caller separates
-  // successive uses of the buffer by a barrier (`sync` first thing on entry)
-  template <bool INV, unsigned ZM = 0u, class Load, class Out, class Sync>
-  __device__ __forceinline__ static void transform(float4* s, const float2* tw, int t, Load& load, Out& out, Sync& sync) {
-    first<INV, ZM>(s, tw, t, load);
-    inner<INV>(s, tw, t, sync);
+  // last stage: out(k, v) for every k (unnormalised)
+  template <bool INV, class Out>
+  __device__ __forceinline__ static void last(float4* s, int t, Out& out) {
     each<N / RL>(t, [&](int b) {
       const float4* p = last_ptr(s, b);
       c2 v[RL];
@@ -436,6 +477,15 @@ struct PairFFT {
 #pragma unroll
       for (int r = 0; r < RL; ++r) out(b + r * (N / RL), v[r]);
     });
+  }
+
+  // transform: out(k, v) for every k (unnormalised); the caller separates
+  // successive uses of the buffer by a barrier (`sync` first thing on entry)
+  template <bool INV, unsigned ZM = 0u, class Load, class Out, class Sync>
+  __device__ __forceinline__ static void transform(float4* s, const float2* tw, int t, Load& load, Out& out, Sync& sync) {
+    first<INV, ZM>(s, tw, t, load);
+    inner<INV>(s, tw, t, sync);
+    last<INV>(s, t, out);
   }
 
   // last stage with the outputs left in the buffer: frequency k = b + r N / RL at last_ptr(b) + r VP
@@ -469,6 +519,20 @@ struct PairFFT {
 #pragma unroll
       for (int r = 0; r < RL; ++r) sstore(p + r * VP, v[r]);
     }
+  }
+  // the second half of a round trip on loaded values, v[r] = load(b + r N / RL): with back() a whole transform
+  // in the operation order of a round trip's way back
+  template <bool INV, class Load>
+  __device__ __forceinline__ static void enter(float4* s, int t, Load& load) {
+    each<N / RL>(t, [&](int b) {
+      float4* p = last_ptr(s, b);
+      c2 v[RL];
+#pragma unroll
+      for (int r = 0; r < RL; ++r) v[r] = load(b + r * (N / RL));
+      PDFT<RL, INV>::run(v);
+#pragma unroll
+      for (int r = 0; r < RL; ++r) sstore(p + r * VP, v[r]);
+    });
   }
   // the way back from the centre: out(n, v), natural order, unnormalised
   template <bool INV, class Out, class Sync>

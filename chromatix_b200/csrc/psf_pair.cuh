@@ -51,8 +51,8 @@ __global__ void __launch_bounds__(PsfPairRows<NX>::THREADS, PsfPairRows<NX>::MIN
     float2* dst = a.T + ((size_t)zl * a.rowsum + a.prefix[w] + r) * a.ldT;
     auto load = [&](int n) -> c2 {
       const int c = add_mod(n, NX / 2, NX) - xlo;  // ifftshift along x, then the box column
-      if ((unsigned)c >= (unsigned)nc) return pzero();
-      return pmul(pmulw<false>(ppack(m[c], m[up + c]), cxz[c]), cy);
+      const bool ok = (unsigned)c < (unsigned)nc;
+      return pmul(pmulw<false>(ppack(ld2z(m + c, ok), ld2z(m + up + c, ok)), ld2z(cxz + c, ok)), cy);
     };
     auto out = [&](int k, c2 v) {
       if (valid) {
@@ -121,8 +121,7 @@ __global__ void __launch_bounds__(PsfPairCols<NY>::THREADS, PsfPairCols<NY>::MIN
       const float2* src = a.T + ((size_t)zl * a.rowsum + a.prefix[w] - a.ylo[w]) * a.ldT + x;
       auto load = [&](int n) -> c2 {
         const int y = add_mod(n, NY / 2, NY);  // ifftshift along y
-        if (!ok || y < slo || y >= shi) return pzero();
-        return ppack(__ldcg(reinterpret_cast<const float4*>(src + (size_t)y * a.ldT)));
+        return ppack(ld4z(src + (size_t)y * a.ldT, ok && y >= slo && y < shi));
       };
       const bool first = w == 0, last = w + 1 == a.W;
       auto out = [&](int k, c2 v) {

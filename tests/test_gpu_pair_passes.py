@@ -120,3 +120,29 @@ def test_psf_stack(ny, nx, wv):
     out = cf.ff_lens(cf.phase_change(f, to_cuda(phase)), 200000.0, 1.33).intensity.cpu().numpy()
     ref = O.ff_lens(O.phase_change(O.objective_point_source(*args, offset=off), phase), 200000.0, 1.33).intensity
     assert O.rel_l2(out, np.asarray(ref).reshape(out.shape)) < 2 * BAR
+
+
+@pytest.mark.parametrize("planes,h,w,kh,kw", [(3, 64, 128, 64, 128), (2, 101, 190, 101, 190), (4, 75, 333, 60, 330),
+                                              (2, 300, 131, 305, 140), (1, 700, 129, 700, 129), (2, 130, 2048, 131, 2047),
+                                              (2, 2048, 130, 2048, 130)])
+def test_convolution_pairs(planes, h, w, kh, kw):
+    """Sample and kernel as a pair: odd numbers of rows (a row of zeros completes the last pair), odd widths (element
+    by element loads), unequal shapes, the longest lengths; per plane and summed.  Four FP32 transforms of each input
+    and products: the propagation's tolerance without the sin / cos, doubled for the sum over planes."""
+    from chromatix_b200.ops import fourier_convolution
+
+    rng = np.random.default_rng(h + w)
+    a = rng.standard_normal((planes, h, w)).astype(np.float32)
+    k = rng.standard_normal((planes, kh, kw)).astype(np.float32)
+    P, Q = h + kh, w + kw
+    F = np.fft.rfft2(a.astype(np.float64), (P, Q)) * np.fft.rfft2(k.astype(np.float64), (P, Q))
+    y0, x0 = (kh - 1) // 2, (kw - 1) // 2
+    ref = np.fft.irfft2(F, (P, Q))[:, y0:y0 + h, x0:x0 + w]
+    out = fourier_convolution(to_cuda(a), to_cuda(k)).cpu().numpy()
+    assert O.rel_l2(out, ref) < BAR
+    red = fourier_convolution(to_cuda(a), to_cuda(k), reduce=True).cpu().numpy()
+    assert O.rel_l2(red, ref.sum(0)) < BAR
+    # one kernel for every plane
+    one = fourier_convolution(to_cuda(a), to_cuda(k[:1])).cpu().numpy()
+    F1 = np.fft.rfft2(a.astype(np.float64), (P, Q)) * np.fft.rfft2(k[:1].astype(np.float64), (P, Q))
+    assert O.rel_l2(one, np.fft.irfft2(F1, (P, Q))[:, y0:y0 + h, x0:x0 + w]) < BAR
