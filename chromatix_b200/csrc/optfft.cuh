@@ -25,6 +25,9 @@ __device__ __forceinline__ float2 chirp(double c, double ry, double rx) {
   return expi_reduced(c * (ry * ry + rx * rx));
 }
 
+// the passes on pairs of rows / columns (optfft_pair.cuh), for lengths with a pair plan
+cx_status opt_dispatch_rows_pair(int n, const float2* u, float2* T, const OptArgs& a, cudaStream_t st);
+cx_status opt_dispatch_cols_pair(int n, const float2* T, float2* out, const OptArgs& a, cudaStream_t st);
 cx_status opt_dispatch_rows(int n, const float2* u, float2* T, const OptArgs& a, cudaStream_t st);
 cx_status opt_dispatch_cols(int n, const float2* T, float2* out, const OptArgs& a, cudaStream_t st);
 }  // namespace cx

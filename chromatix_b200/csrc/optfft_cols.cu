@@ -1,5 +1,6 @@
 // Column pass of the chirped optical FFT (see optfft.cuh).
 #include "optfft.cuh"
+#include "pair_fft.cuh"
 
 namespace cx {
 
@@ -73,11 +74,12 @@ static cx_status launch_opt_cols(const float2* T, float2* out, const OptArgs& a,
 }
 
 cx_status opt_dispatch_cols(int n, const float2* T, float2* out, const OptArgs& a, cudaStream_t st) {
+  if (pair_length(n)) return opt_dispatch_cols_pair(n, T, out, a, st);
   switch (n) {
 #define CX_CASE_(N) \
   case N:           \
     return launch_opt_cols<N>(T, out, a, st);
-    CX_FOR_EACH_SIZE(CX_CASE_)
+    CX_FOR_EACH_SHORT_SIZE(CX_CASE_)
 #undef CX_CASE_
   }
   set_error("FFT length %d is not supported", n);

@@ -1,5 +1,6 @@
 // Row pass of the chirped optical FFT (see optfft.cuh).
 #include "optfft.cuh"
+#include "pair_fft.cuh"
 
 namespace cx {
 
@@ -59,11 +60,12 @@ static cx_status launch_opt_rows(const float2* u, float2* T, const OptArgs& a, c
 }
 
 cx_status opt_dispatch_rows(int n, const float2* u, float2* T, const OptArgs& a, cudaStream_t st) {
+  if (pair_length(n)) return opt_dispatch_rows_pair(n, u, T, a, st);
   switch (n) {
 #define CX_CASE_(N) \
   case N:           \
     return launch_opt_rows<N>(u, T, a, st);
-    CX_FOR_EACH_SIZE(CX_CASE_)
+    CX_FOR_EACH_SHORT_SIZE(CX_CASE_)
 #undef CX_CASE_
   }
   set_error("FFT length %d is not supported", n);
