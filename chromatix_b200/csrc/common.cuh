@@ -142,6 +142,14 @@ __device__ __forceinline__ bool bulk_wait(uint64_t* bar, unsigned phase, int pol
   return false;
 }
 
+// Programmatic dependent launch: let the next kernel of the stream start its
+// prologue, and wait for the previous kernel's results.  A prologue (what runs
+// before pdl_wait) touches only data that was complete before a kernel
+// launched without the attribute: a kernel may start before its predecessor's
+// predecessor has finished.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Cast helpers that block FMA contraction, for the float32 reference-order
 // evaluation mode.
 __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }

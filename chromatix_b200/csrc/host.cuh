@@ -301,4 +301,20 @@ inline cudaError_t set_smem(K kernel, size_t smem) {
   return cudaSuccess;  // done once by kernel_facts (called by persistent_grid before every launch)
 }
 
+// launch, with `pdl` as a programmatic dependent of the stream's previous kernel (see pdl_wait)
+template <class K, class... Args>
+inline cudaError_t launch_kernel(K kernel, int grid, int threads, size_t smem, cudaStream_t st, bool pdl, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 }  // namespace cx

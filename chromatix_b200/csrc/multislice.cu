@@ -42,7 +42,12 @@ static cx_status ms_plan(const cx_ms_desc* d, MsPlan* p) {
   }
   p->D = d->n_slices;
   int K = d->checkpoint_every;
-  if (K <= 0) K = (int)std::ceil(std::sqrt((double)p->D));
+  // by default every slice's field is kept where the stack of them takes at most 4 GiB (no recomputation: 128
+  // slices of 1024^2 with gradient 7.4 -> 5.8 ms), else a checkpoint every sqrt(D) slices
+  if (K <= 0)
+    K = (double)(p->D + 1) * p->py * p->px * sizeof(float2) <= 4.0 * 1024 * 1024 * 1024
+            ? p->D
+            : (int)std::ceil(std::sqrt((double)p->D));
   if (K > p->D) K = p->D;
   p->K = K;
   p->nseg = (p->D + K - 1) / K;
@@ -79,11 +84,11 @@ static cx_status ms_plan(const cx_ms_desc* d, MsPlan* p) {
 static size_t al(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // workspace: [planes (4 x cx_plane)] [H table] [F state] ([G state] [2 x K records] for the adjoint:
-// the records of two segments, one being read by the adjoint while the next is recomputed)
+// the records of up to two recomputed segments, one being read by the adjoint while the next is recomputed)
 static size_t ms_ws(const MsPlan& p, bool grad) {
   const size_t field = sizeof(float2) * (size_t)p.py * p.px;
   size_t b = al(4 * sizeof(cx_plane)) + 2 * al(field);
-  if (grad) b += al(field) + 2 * (size_t)p.K * al(field);
+  if (grad) b += al(field) + (size_t)(p.nseg > 2 ? 2 : p.nseg - 1) * p.K * al(field);
   return b;
 }
 
@@ -117,7 +122,9 @@ static MsArgs ms_args(const cx_ms_desc* d, const MsPlan& p) {
   a.precision = d->precision;
   a.lam = d->wavelength;
   a.dz = d->dz;
-  a.kdz_f = (float)(6.283185307179586476925286766559 * d->dz / d->wavelength);
+  const double kdz = 6.283185307179586476925286766559 * d->dz / d->wavelength;
+  a.kdz_f = (float)kdz;
+  a.kdz_lo = (float)(kdz - (double)a.kdz_f);
   a.twg = p.col.twg;
   a.load_scale = 1.f;
   return a;
@@ -169,6 +176,7 @@ static cx_status col_pass(const MsPlan& p, const cx_plane* plane, float2* buf, d
     a.kernel = CX_KERNEL_EXPLICIT;
     a.H = Htab;
     a.conj_h = conj_h ? 1 : 0;
+    a.pdl = 1;
   } else {
     a.bandlimit = 0;
     a.remove_evanescent = 0;

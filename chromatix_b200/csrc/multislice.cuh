@@ -30,6 +30,7 @@ struct MsArgs {
   int mode, precision, slice, record;
   double lam, dz;
   float kdz_f;          // 2 pi dz / lam rounded once to float
+  float kdz_lo;         // and what the rounding left
   int sy, sx, oy, ox;   // MS_LOAD source: (sy, sx) matrix placed at offset (oy, ox) of the padded grid
   const float* dn;      // (D, ny, nx) refractive-index change (unpadded)
   const float* ab;      // (D, ny, nx) absorption (unpadded)
@@ -258,6 +259,8 @@ __global__ void __launch_bounds__(RowCfg<NX>::THREADS, RowCfg<NX>::MINB) k_ms_ro
   }
 }
 
+// the passes on row pairs (multislice_pair.cuh), for lengths with a pair plan
+cx_status ms_dispatch_rows_pair(int n, const MsArgs& a, cudaStream_t st);
 cx_status ms_dispatch_rows(int n, const MsArgs& a, cudaStream_t st);
 // CX_PREC_SPLIT16 row passes on the tensor cores (multislice_tc.cu) where the
 // padded row length is compiled in; other lengths and the fluorescent step

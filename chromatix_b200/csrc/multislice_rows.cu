@@ -1,5 +1,6 @@
 // Row passes of the multislice loop (see multislice.cuh).
 #include "multislice.cuh"
+#include "pair_fft.cuh"
 
 namespace cx {
 
@@ -33,11 +34,12 @@ static cx_status launch_ms_rows(const MsArgs& a, cudaStream_t st) {
 }
 
 cx_status ms_dispatch_rows(int n, const MsArgs& a, cudaStream_t st) {
+  if (pair_length(n)) return ms_dispatch_rows_pair(n, a, st);
   switch (n) {
 #define CX_CASE_(N) \
   case N:           \
     return launch_ms_rows<N>(a, st);
-    CX_FOR_EACH_SIZE(CX_CASE_)
+    CX_FOR_EACH_SHORT_SIZE(CX_CASE_)
 #undef CX_CASE_
   }
   set_error("FFT length %d is not supported", n);

@@ -26,6 +26,7 @@ struct Prop2DArgs {
   double na_f2;  // >= 0: k-space NA mask |f|^2 <= na_f2 (samples.py:276-280); < 0: none
   int precise;   // 1: FP64 sin/cos (tables reused many times); 0: FP64 reduction + hardware sin/cos
   int conj_h;    // 1: use conj(H) (adjoint passes; any kernel kind)
+  int pdl = 0;   // 1: the table column pass may start beside its predecessor (H complete before that one's)
   const cx_plane* planes;
   const float2* H;
   const float2* twg;  // device twiddle tables (ensure_twiddles)

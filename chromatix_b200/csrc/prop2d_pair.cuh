@@ -15,10 +15,10 @@
 namespace cx {
 
 // first-stage inputs that a field in the central half of the padded axis leaves zero
-template <int N>
+template <int N, bool LONE = false>
 constexpr unsigned pair_band_mask() {
   unsigned m = 0u;
-  constexpr int R = PairPlan<N>::R1;
+  constexpr int R = PairPlan<N, LONE>::R1;
   for (int r = 0; r < R; ++r)
     if (r < R / 4 || r >= 3 * R / 4) m |= 1u << r;
   return m;
@@ -129,21 +129,22 @@ __global__ void __launch_bounds__(PairRows<NX>::THREADS, PairRows<NX>::MINB)
 // shared memory beside the tile's loads.
 template <int NY, bool TABLE>
 struct PropPairCols {
-  static constexpr int L = PairPlan<NY>::L;
+  using P = PairPlan<NY, TABLE>;
+  static constexpr int L = P::L;
   static constexpr int HROWS = TABLE ? NY : NY / 2 + 1;
   static constexpr size_t bytes(int vp) {
-    return sizeof(float4) * (size_t)vp * (PairPlan<NY>::R1 * (NY / PairPlan<NY>::R1 + 1) + HROWS);
+    return sizeof(float4) * (size_t)vp * (P::R1 * (NY / P::R1 + 1) + HROWS);
   }
   // the widest tile of at most 512 lanes with two CTAs per SM; two column
-  // pairs (whole 32-byte sectors) where one CTA per SM has room for them.  With a table (the multislice loop, one
-  // plane at a time: fewer tiles than SMs) one CTA per SM is enough for any width.
+  // pairs (whole 32-byte sectors) where one CTA per SM has room for them.  With a table (the multislice loop, whose
+  // adjoint runs two chains of one-plane passes side by side) three CTAs per SM.
   static constexpr int vp() {
     int v = 4;
-    while (v > 1 && (v * L > 512 || bytes(v) > (TABLE || v == 2 ? 200 : 104) * 1024)) v /= 2;
+    while (v > 1 && (v * L > 512 || bytes(v) > (v == 2 ? 200 : (TABLE ? 74 : 104)) * 1024)) v /= 2;
     return v;
   }
   static constexpr int VP = vp();
-  using F = PairFFT<NY, VP>;
+  using F = PairFFT<NY, VP, TABLE>;
   static constexpr int THREADS = VP * L;
   static constexpr int TWB = (F::TW * (int)sizeof(float2) + 15) & ~15;
   static constexpr size_t H_OFF = TWB + sizeof(float4) * (size_t)F::ELEMS;
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(PropPairCols<NY, TABLE>::THREADS, PropPairCols
   using F = typename C::F;
   constexpr int VP = C::VP, V = 2 * VP;
   extern __shared__ __align__(16) char smem[];
+  if constexpr (TABLE) pdl_trigger();
   float2* tw = reinterpret_cast<float2*>(smem);
   float4* s0 = reinterpret_cast<float4*>(smem + C::TWB);
   float4* hs = reinterpret_cast<float4*>(smem + C::H_OFF);
@@ -195,10 +197,10 @@ __global__ void __launch_bounds__(PropPairCols<NY, TABLE>::THREADS, PropPairCols
     const float2* src = T + (size_t)pl.in_plane * a.ny * a.px + x;
     auto load = [&](int n) -> c2 {
       const int r = n - a.pad_y;
-      if (!ok0 || (unsigned)r >= (unsigned)a.ny) return pzero();
-      const float2* p = src + (size_t)r * a.px;
-      if constexpr (VEC) return ppack(*reinterpret_cast<const float4*>(p));
-      return ppack(p[0], ok1 ? p[1] : make_float2(0.f, 0.f));
+      const bool ok = ok0 && (unsigned)r < (unsigned)a.ny;
+      const float2* p = src + (ptrdiff_t)r * a.px;
+      if constexpr (VEC) return ppack(ld4z(p, ok));
+      return ppack(ld2z(p, ok), ld2z(p + 1, ok && ok1));
     };
     __syncthreads();  // the previous tile (and its propagator) has been read
     const float2* Hp = TABLE ? a.H + (size_t)pl.h_plane * NY * a.px : nullptr;
@@ -219,8 +221,11 @@ __global__ void __launch_bounds__(PropPairCols<NY, TABLE>::THREADS, PropPairCols
         }
       }
     }
+    if constexpr (TABLE) {
+      if (o == o0) pdl_wait();  // the table and the twiddles are on their way
+    }
     if (band)
-      F::template first<false, pair_band_mask<NY>()>(s, tw, t, load);
+      F::template first<false, pair_band_mask<NY, TABLE>()>(s, tw, t, load);
     else
       F::template first<false>(s, tw, t, load);
     if constexpr (TABLE) {
@@ -327,8 +332,7 @@ static cx_status launch_cols_pair(const float2* T, float2* T2, const Prop2DArgs&
   long per = items / (4 * resident);
   per = per < 1 ? 1 : (per > 8 ? 8 : per);
   const long grid = tiles * ((a.n_out_planes + per - 1) / per);
-  k<<<(unsigned)grid, C::THREADS, C::SMEM, st>>>(T, T2, a, (int)per);
-  CX_LAUNCH_CHECK();
+  CX_CUDA_TRY(launch_kernel(k, (int)grid, C::THREADS, C::SMEM, st, TABLE && a.pdl, T, T2, a, (int)per));
   return CX_OK;
 }
 

@@ -223,7 +223,8 @@ def multislice_thick_sample(field: Field, absorption_stack, dn_stack, n, thickne
     with an optional NA mask, and cropped by ``pad_width``.  Differentiable with
     respect to the field, ``dn_stack`` and ``absorption_stack`` through a
     hand-written adjoint that stores a checkpoint every ``checkpoint_every``
-    slices (default ceil(sqrt(D))) and recomputes in between.
+    slices (default: every slice where the padded fields take at most 4 GiB, else
+    ceil(sqrt(D))) and recomputes in between.
     """
     from .. import config
     from .sources import materialize

@@ -266,7 +266,7 @@ typedef struct {
   int32_t n_slices;          /* D */
   int32_t precision;         /* cx_precision */
   int32_t remove_evanescent, bandlimit;  /* slice propagator options */
-  int32_t checkpoint_every;  /* K; <= 0: ceil(sqrt(D)) */
+  int32_t checkpoint_every;  /* K; <= 0: D where D + 1 padded planes take at most 4 GiB, else ceil(sqrt(D)) */
   double n_medium, wavelength, dy, dx;
   double dz;                 /* thickness_per_slice */
   double reverse_distance;   /* defocus back by this distance */
