@@ -395,6 +395,11 @@ __global__ void __launch_bounds__(MbsXCfg<NX>::THREADS, MbsXCfg<NX>::MINB) k_mbs
   }
 }
 
+// the strided passes on column pairs (mbs_pair.cuh), for lengths and states that mbs_on_pairs accepts
+bool mbs_on_pairs(int n, const MbsArgs& a);
+cx_status mbs_dispatch_cols_pair(int n, bool inv, const MbsArgs& a, long n_outer, int inner, long ostride, long E,
+                                 cudaStream_t st);
+cx_status mbs_dispatch_x_pair(int n, const MbsArgs& a, cudaStream_t st);
 cx_status mbs_dispatch_z(int n, int mode, const MbsArgs& a, cudaStream_t st);
 cx_status mbs_dispatch_cols(int n, bool inv, const MbsArgs& a, long n_outer, int inner, long ostride, long E,
                             cudaStream_t st);

@@ -82,6 +82,7 @@ cx_status mbs_dispatch_z(int n, int mode, const MbsArgs& a, cudaStream_t st) {
 
 cx_status mbs_dispatch_cols(int n, bool inv, const MbsArgs& a, long n_outer, int inner, long ostride, long E,
                             cudaStream_t st) {
+  if (mbs_on_pairs(n, a)) return mbs_dispatch_cols_pair(n, inv, a, n_outer, inner, ostride, E, st);
   switch (n) {
 #define CX_CASE_(N)                                                                       \
   case N:                                                                                 \
@@ -95,6 +96,7 @@ cx_status mbs_dispatch_cols(int n, bool inv, const MbsArgs& a, long n_outer, int
 }
 
 cx_status mbs_dispatch_x(int n, const MbsArgs& a, cudaStream_t st) {
+  if (mbs_on_pairs(n, a)) return mbs_dispatch_x_pair(n, a, st);
   switch (n) {
 #define CX_CASE_(N) \
   case N:           \

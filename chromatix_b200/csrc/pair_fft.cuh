@@ -546,6 +546,10 @@ struct PairFFT {
       mid2<INV, true>(s, tw, t);
       sync();
     }
+    back_last<INV>(s, tw, t, out);
+  }
+  template <bool INV, class Out>
+  __device__ __forceinline__ static void back_last(float4* s, const float2* tw, int t, Out& out) {
     each<M>(t, [&](int j) {
       c2 v[R1];
 #pragma unroll

@@ -146,3 +146,84 @@ def test_convolution_pairs(planes, h, w, kh, kw):
     one = fourier_convolution(to_cuda(a), to_cuda(k[:1])).cpu().numpy()
     F1 = np.fft.rfft2(a.astype(np.float64), (P, Q)) * np.fft.rfft2(k[:1].astype(np.float64), (P, Q))
     assert O.rel_l2(one, np.fft.irfft2(F1, (P, Q))[:, y0:y0 + h, x0:x0 + w]) < BAR
+
+
+@pytest.mark.parametrize("ny,nx,pad,wv", [(128, 160, (0, 0), 1), (192, 6, (0, 0), 2), (224, 5, (0, 0), 1), (256, 320, (64, 32), 3),
+                                          (320, 10, (32, 1), 1), (2048, 10, (0, 0), 2)])
+def test_optical_fft_passes(ny, nx, pad, wv):
+    """The chirped optical FFT on pairs: plain (ff_lens with a pupil, inverse lens), with an output chirp (df_lens),
+    with chirps, padding and crop (transform_propagate); two transforms and FP64-reduced chirps."""
+    import chromatix_b200.functional as cf
+
+    rng = np.random.default_rng(ny + nx)
+    lam = np.array([0.532, 0.45, 0.63][:wv])
+    spec = lam if wv > 1 else float(lam[0])
+    u = _crand(rng, (2, ny, nx) + ((wv,) if wv > 1 else ()))
+    f = _field(u, dx=1.1, lam=spec)
+    calls = [lambda m, g: m.ff_lens(g, 500.0, 1.33, NA=0.05), lambda m, g: m.ff_lens(g, 500.0, 1.33, inverse=True),
+             lambda m, g: m.df_lens(g, 420.0, 500.0, 1.33), lambda m, g: m.transform_propagate(g, 3000.0, 1.0, pad)]
+    for i, call in enumerate(calls):
+        out = call(cf, f).u.cpu().numpy()
+        for b in range(2):
+            ref = call(O, O.field_build(u[b], 1.1, spec)).u
+            assert O.rel_l2(out[b], np.asarray(ref).reshape(out[b].shape)) < BAR, (i, b)
+
+
+@pytest.mark.parametrize("n,pad,slices", [(128, 0, 5), (130, 15, 4), (100, 14, 3), (224, 0, 3), (320, 32, 3), (448, 0, 2),
+                                          (1024, 0, 2), (1280, 0, 2), (2048, 0, 1)])
+def test_multislice_rows(n, pad, slices):
+    """The slice loop's row passes on pairs: sides that 4 does not divide (rows read element by element), padding,
+    with and without recomputation.  Each slice adds two transforms each way; gradients within twice the field's bar."""
+    import torch
+
+    import chromatix_b200.functional as cf
+
+    if n + 2 * pad not in LENGTHS:
+        pad = (min(m for m in LENGTHS if m > n + 2 * pad) - n) // 2
+    rng = np.random.default_rng(n)
+    dn = (0.02 * rng.standard_normal((slices, n, n))).astype(np.float32)
+    ab = rng.uniform(0, 0.01, (slices, n, n)).astype(np.float32)
+    u = _crand(rng, (n, n))
+    bar = BAR * (1 + slices)
+    ref = O.multislice_thick_sample(O.field_build(u, 0.15, 0.532), ab, dn, 1.33, 0.3, pad, NA=0.9).u
+    f = _field(u, dx=0.15)
+    d = to_cuda(dn).requires_grad_(True)
+    out = cf.multislice_thick_sample(f, to_cuda(ab), d, 1.33, 0.3, pad, NA=0.9)
+    assert O.rel_l2(out.u.detach().cpu().numpy(), np.asarray(ref).reshape(n, n)) < bar
+    g = to_cuda(_crand(rng, (n, n)))
+    (g0,) = torch.autograd.grad(out.u, d, g)
+    d1 = to_cuda(dn).requires_grad_(True)
+    (g1,) = torch.autograd.grad(cf.multislice_thick_sample(f, to_cuda(ab), d1, 1.33, 0.3, pad, NA=0.9, checkpoint_every=1).u, d1, g)
+    assert torch.equal(g0, g1)
+    # dL/d dn of the FP64 recursion, along one direction
+    if pad == 0:
+        w = rng.standard_normal(dn.shape).astype(np.float32)
+        h = 1e-3
+        gc = g.cpu().numpy().astype(np.complex128)
+        L = [np.sum((gc.conj() * np.asarray(O.multislice_thick_sample(O.field_build(u, 0.15, 0.532), ab, dn + s * h * w, 1.33,
+                                                                     0.3, 0, NA=0.9).u).reshape(n, n)).real) for s in (1, -1)]
+        got = float(np.sum(g0.cpu().numpy().astype(np.float64) * w))
+        assert abs(got - (L[0] - L[1]) / (2 * h)) < 1e-4 * np.linalg.norm(w) * float(torch.linalg.vector_norm(g0)) / np.sqrt(w.size) + 1e-2 * abs(got)
+
+
+@pytest.mark.parametrize("n", [128, 160, 192, 224, 256, 320, 384, 448, 512])
+@pytest.mark.parametrize("axis", [0, 1])
+def test_mbs_strided_passes(n, axis):
+    """One update of the modified Born series with one long strided axis (x: three components and the k-space
+    operator; y), ragged tiles (20 columns) against the FP64 restatement: six transforms and the operator's
+    reciprocals, eight FP32 roundings of the state."""
+    import torch
+
+    from chromatix_b200.experimental import mbs
+
+    shape = (n, 16, 20) if axis == 0 else (16, n, 20)
+    rng = np.random.default_rng(n)
+    k0, sp = 2 * np.pi / 0.5, 0.1
+    eps = 1.0 + 0.3 * rng.uniform(size=shape) + 0.02j * rng.uniform(size=shape)
+    src = _crand(rng, shape + (3,))
+    op = O.MBSOperator(eps.astype(np.complex64).astype(np.complex128), sp, k0, src.astype(np.complex128))
+    sample = mbs.Sample(to_cuda(eps.astype(np.complex64)), sp)
+    source = mbs.Source(torch.zeros(shape + (3,), dtype=torch.complex64, device="cuda"), k0)
+    source.field = to_cuda(src)
+    E = mbs.solve(sample, source, maxiter=1, tol=0.0, shift=op.bias, scale=op.scale).cpu().numpy()
+    assert O.rel_l2(E, op.step(op.prec_y) * op.num_scale) < 2 * BAR
