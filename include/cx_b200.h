@@ -594,7 +594,8 @@ cx_status cx_plane_wave(const cx_ew_desc* d, const double* wv_params_dev, double
 /* The Fourier multiplier of kernel_propagate (functional/propagation.py:391-394)
  * for grids the fused passes do not cover (their transforms are chirp-Z passes):
  * out[b, y, x, w] = u[b, y, x, w] H[b n_wv + w, y, x], conj(H) when conj_h; H
- * planar (n_batch n_wv, ny, nx) as cx_fill_propagator writes it. */
+ * planar (n_batch n_wv, ny, nx) as cx_fill_propagator writes it, or, with
+ * map_batched = -1, (n_wv, ny, nx) for every batch element. */
 cx_status cx_cmul_planar(const cx_ew_desc* d, const void* u, const void* H, int32_t conj_h, void* out,
                          cx_stream_t stream);
 /* Pupils (functional/pupils.py:17-67) on the field grid g = d_w (i - N/2) + origin:
