@@ -153,6 +153,9 @@ __global__ void __launch_bounds__(ColCfg<L>::THREADS, ColCfg<L>::MINB) k_czt_col
   }
 }
 
+// the passes on pairs of vectors (czt_pair.cuh), for lengths with a pair plan
+cx_status czt_dispatch_rows_pair(int L, const CztArgs& a, cudaStream_t st);
+cx_status czt_dispatch_cols_pair(int L, const CztArgs& a, cudaStream_t st);
 cx_status czt_dispatch_rows(int L, const CztArgs& a, cudaStream_t st);
 cx_status czt_dispatch_cols(int L, const CztArgs& a, cudaStream_t st);
 

@@ -1,5 +1,6 @@
 // Chirp-Z transform along a strided axis, column tiles (see czt.cuh).
 #include "czt.cuh"
+#include "pair_fft.cuh"
 
 namespace cx {
 
@@ -14,11 +15,13 @@ static cx_status launch_czt_cols(const CztArgs& a, cudaStream_t st) {
 }
 
 cx_status czt_dispatch_cols(int L, const CztArgs& a, cudaStream_t st) {
+  if (pair_length(L)) return czt_dispatch_cols_pair(L, a, st);
   switch (L) {
 #define CX_CASE_(N) \
   case N:           \
     return launch_czt_cols<N>(a, st);
-    CX_FOR_EACH_1D_SIZE(CX_CASE_)
+    CX_FOR_EACH_SHORT_SIZE(CX_CASE_)
+    CX_FOR_EACH_CZT_LONG_SIZE(CX_CASE_)
 #undef CX_CASE_
   }
   set_error("FFT length %d is not supported", L);

@@ -1,5 +1,6 @@
 // Chirp-Z transform, one team per vector (see czt.cuh).
 #include "czt.cuh"
+#include "pair_fft.cuh"
 
 namespace cx {
 
@@ -14,11 +15,13 @@ static cx_status launch_czt_rows(const CztArgs& a, cudaStream_t st) {
 }
 
 cx_status czt_dispatch_rows(int L, const CztArgs& a, cudaStream_t st) {
+  if (pair_length(L)) return czt_dispatch_rows_pair(L, a, st);
   switch (L) {
 #define CX_CASE_(N) \
   case N:           \
     return launch_czt_rows<N>(a, st);
-    CX_FOR_EACH_1D_SIZE(CX_CASE_)
+    CX_FOR_EACH_SHORT_SIZE(CX_CASE_)
+    CX_FOR_EACH_CZT_LONG_SIZE(CX_CASE_)
 #undef CX_CASE_
   }
   set_error("FFT length %d is not supported", L);

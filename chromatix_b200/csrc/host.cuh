@@ -43,7 +43,8 @@ void set_error(const char* fmt, ...);
 // Longer lengths compiled only for the 1D transform (cx_fft1d) and the
 // chirp-Z passes, whose Bluestein length reaches n + m - 1 (up to 8192 for a
 // 4096-point input): 2^9 3^2, 2^10 5, 2^11 3, 2^10 7, 2^13.
-#define CX_FOR_EACH_LONG_SIZE(X) X(4608) X(5120) X(6144) X(7168) X(8192)
+#define CX_FOR_EACH_CZT_LONG_SIZE(X) X(4608) X(5120) X(6144) X(7168)
+#define CX_FOR_EACH_LONG_SIZE(X) CX_FOR_EACH_CZT_LONG_SIZE(X) X(8192)
 #define CX_FOR_EACH_1D_SIZE(X) CX_FOR_EACH_SIZE(X) CX_FOR_EACH_LONG_SIZE(X)
 // The Fourier-multiplier propagation passes also take 8192 (a 4096^2 field
 // padded by 2048 per side, the reference's high-resolution band-limited ASM

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(MbsPairCfg<N, 3>::THREADS, MbsPairCfg<N, 3>::M
     const float2 kz = make_float2(a.kfz * (float)freq_index(iz, a.Z), a.kfz * (float)freq_index(iz + 1, a.Z));
     const float2 kyz = make_float2(ky * ky + kz.x * kz.x, ky * ky + kz.y * kz.y);
     __syncthreads();  // the previous tile has been read
-#pragma unroll 1
+#pragma unroll
     for (int m = 0; m < 3; ++m) {
       const float2* base = a.buf + (size_t)m * a.vox + cc;
       auto load = [&](int j) -> c2 { return ppack(ld4z(base + (long)j * inner, ok)); };
