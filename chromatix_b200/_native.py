@@ -258,9 +258,18 @@ def torch_mod():
     return torch
 
 
-def stream_handle(device=None) -> int:
+def device_index(device=None) -> int:
+    """CUDA index of ``device`` (a torch.device, a string or None: the current one)."""
     torch = torch_mod()
-    return torch.cuda.current_stream(device).cuda_stream
+    if isinstance(device, (str, int)):
+        device = torch.device(device)
+    i = None if device is None else device.index
+    return torch.cuda.current_device() if i is None else i
+
+
+def stream_handle(device=None) -> int:
+    """cudaStream_t of the current stream (without building a torch.cuda.Stream)."""
+    return torch_mod()._C._cuda_getCurrentRawStream(device_index(device))
 
 
 def ptr(t) -> int:
@@ -281,35 +290,49 @@ def upload(arr: np.ndarray, device):
     return t.to(device, non_blocking=True)
 
 
-# (descriptor type and bytes, plane table bytes, device) -> (workspace bytes,
-# device plane table, event after its upload): repeated calls with the same
+# (descriptor type and bytes, plane table bytes, device) -> [workspace bytes,
+# device plane table, event after its upload]: repeated calls with the same
 # geometry skip the workspace query and the host-to-device copy of their
-# plane table.  The device tables are read-only; a call on another stream
-# waits for the upload's event before its kernels read the table.
+# plane table.  The device tables are read-only; a call waits for the upload's
+# event before its kernels read the table, until the event has been seen done.
 _TABLES = collections.OrderedDict()
 _TABLES_SIZE = 128
+
+
+def _table(key, arr, device, ws_query=None):
+    torch = torch_mod()
+    hit = _TABLES.get(key)
+    if hit is not None:
+        _TABLES.move_to_end(key)
+        ev = hit[2]
+        if ev is not None and not torch.cuda.is_current_stream_capturing():
+            if ev.query():
+                hit[2] = None
+            else:
+                torch.cuda.current_stream(device).wait_event(ev)
+        return hit
+    ws_bytes = int(ws_query()) if ws_query is not None else 0
+    table = upload(arr, device)
+    ev = torch.cuda.Event()
+    ev.record(torch.cuda.current_stream(device))
+    hit = _TABLES[key] = [ws_bytes, table, ev]
+    if len(_TABLES) > _TABLES_SIZE:
+        _TABLES.popitem(last=False)
+    return hit
 
 
 def device_table(desc, planes: np.ndarray, device, ws_query):
     """(workspace bytes, device copy of ``planes``) for a launch described by
     the ctypes struct ``desc``; ``ws_query(desc)`` returns the workspace size."""
-    torch = torch_mod()
-    key = (type(desc).__name__, ctypes.string_at(ctypes.addressof(desc), ctypes.sizeof(desc)), planes.tobytes(),
-           device.index)
-    hit = _TABLES.get(key)
-    if hit is not None:
-        _TABLES.move_to_end(key)
-        if not torch.cuda.is_current_stream_capturing():
-            torch.cuda.current_stream(device).wait_event(hit[2])
-        return hit[0], hit[1]
-    ws_bytes = int(ws_query(desc))
-    table = to_device_bytes(planes, device)
-    ev = torch.cuda.Event()
-    ev.record(torch.cuda.current_stream(device))
-    _TABLES[key] = (ws_bytes, table, ev)
-    if len(_TABLES) > _TABLES_SIZE:
-        _TABLES.popitem(last=False)
-    return ws_bytes, table
+    key = (type(desc).__name__, bytes(desc), planes.tobytes(), device_index(device))
+    hit = _table(key, np.ascontiguousarray(planes).view(np.uint8).reshape(-1), device, lambda: ws_query(desc))
+    return hit[0], hit[1]
+
+
+def constant(arr: np.ndarray, device):
+    """Device copy of a small read-only host array (per-wavelength factors, densities), kept by its content."""
+    key = ("constant", arr.dtype.str, arr.shape, arr.tobytes(), device_index(device))
+    return _table(key, arr, device)[1]
 
 
 def to_device_bytes(arr: np.ndarray, device):

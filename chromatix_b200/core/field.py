@@ -104,7 +104,7 @@ def _intensity(u, C: int, density, out_shape):
     torch = _torch()
     nat.require_cuda(u, "Field.u")
     u = u.to(torch.complex64).contiguous()
-    dens = nat.upload(np.asarray(density, np.float64).reshape(-1), u.device)
+    dens = nat.constant(np.asarray(density, np.float64).reshape(-1), u.device)
     if nat.wants_grad(u):
         return _intensity_fn().apply(u, C, dens, tuple(out_shape))
     return _intensity_launch(u, C, dens, tuple(out_shape))
@@ -557,6 +557,8 @@ def crop(field: Field, crop_width) -> Field:
 
 def shift_grid(field: Field, shift_yx) -> Field:
     """``shift_grid`` (core/field.py:573-585): sets the origin."""
+    if type(shift_yx) is tuple and len(shift_yx) == 2 and np.shape(field.origin) in ((), (1,), (2,)):
+        return field.replace(origin=np.array(shift_yx, dtype=np.float64))
     s = np.atleast_1d(np.asarray(shift_yx, dtype=np.float64))
     if s.size < 2:
         s = np.array([s[0], s[0]])

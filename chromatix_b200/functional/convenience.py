@@ -8,6 +8,8 @@ the store.
 
 from __future__ import annotations
 
+import collections
+
 import numpy as np
 
 from .. import _native as nat
@@ -96,8 +98,14 @@ class _OptPlan:
 
     def __init__(self, desc, planes, in_shape, out_shape):
         self.desc, self.planes, self.in_shape, self.out_shape = desc, planes, tuple(in_shape), tuple(out_shape)
+        self._adjoint = None
 
     def adjoint(self) -> "_OptPlan":
+        if self._adjoint is None:
+            self._adjoint = self._build_adjoint()
+        return self._adjoint
+
+    def _build_adjoint(self) -> "_OptPlan":
         d = cx_optfft_desc.from_buffer_copy(self.desc)
         Py, Px = d.ny + 2 * d.pad_y, d.nx + 2 * d.pad_x
         d.ny, d.nx = Py - 2 * d.crop_y, Px - 2 * d.crop_x
@@ -150,6 +158,15 @@ def _opt_fn():
     return _OPT_FN
 
 
+# optical FFT call parameters -> (plan, output spacing): plans are never modified after they are built
+_OPT_PLANS = collections.OrderedDict()
+_OPT_PLANS_SIZE = 64
+
+
+def _host_bytes(v):
+    return None if v is None else np.asarray(v).tobytes()
+
+
 def run_optfft(field: Field, z: float, n: float, pad_width=(0, 0), crop_width=(0, 0), post=1.0 + 0j,
                chirp_in=None, chirp_out=None, pupil_D=None, precision=None):
     """Launch the chirped optical FFT; returns (u_out, du (wv, 2))."""
@@ -157,6 +174,14 @@ def run_optfft(field: Field, z: float, n: float, pad_width=(0, 0), crop_width=(0
     prec = precision or config.get_precision()
     py_, px_ = pad_width
     cy, cx = crop_width
+    key = (type(field), tuple(field.u.shape), np.shape(field.dx), _host_bytes(field.dx), np.shape(field.origin),
+           _host_bytes(field.origin), _host_bytes(field.spectrum.wavelength), z, n, py_, px_, cy, cx,
+           np.shape(post), _host_bytes(post), _host_bytes(chirp_in), _host_bytes(chirp_out), pupil_D, prec)
+    hit = _OPT_PLANS.get(key)
+    if hit is not None:
+        _OPT_PLANS.move_to_end(key)
+        plan, du = hit
+        return (_opt_fn().apply(field.u, plan) if nat.wants_grad(field.u) else _launch_optfft(plan, field.u)), du.copy()
     ny, nx = field.spatial_shape
     Py, Px = ny + 2 * py_, nx + 2 * px_
     W = field.n_wv
@@ -195,11 +220,14 @@ def run_optfft(field: Field, z: float, n: float, pad_width=(0, 0), crop_width=(0
     oy, ox = Py - 2 * cy, Px - 2 * cx
     out_shape = tuple(B) + (oy, ox) + ((W,) if field.chromatic else ())
     plan = _OptPlan(d, planes, tuple(field.u.shape), out_shape)
+    du = np.stack([nm[2] for nm in norms])
+    _OPT_PLANS[key] = (plan, du.copy())
+    if len(_OPT_PLANS) > _OPT_PLANS_SIZE:
+        _OPT_PLANS.popitem(last=False)
     if nat.wants_grad(field.u):
         u_out = _opt_fn().apply(field.u, plan)
     else:
         u_out = _launch_optfft(plan, field.u)
-    du = np.stack([nm[2] for nm in norms])
     return u_out, du
 
 

@@ -107,7 +107,7 @@ def phase_change(field: Field, phase, spectrally_modulate: bool = True) -> Field
     nat.require_cuda(field.u, "Field.u")
     ph, batched = real_map(field, phase, "phase")
     mod = field.spectrum.spectral_modulation if (spectrally_modulate and field.chromatic) else np.ones(field.n_wv)
-    s = torch.as_tensor(channel_scale(field, mod), device=field.device)
+    s = nat.constant(channel_scale(field, mod), field.device)
     u = field.u.to(torch.complex64).contiguous()
     d = _ew_desc(field, batched)
     if nat.wants_grad(u, ph):

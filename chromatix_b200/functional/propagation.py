@@ -10,6 +10,7 @@ IFFT, the crop in the last FFT's store.
 from __future__ import annotations
 
 import collections
+import functools
 from typing import Literal
 
 import numpy as np
@@ -197,6 +198,7 @@ def _apply_prop(plan: _PropPlan, u):
     return _launch_prop2d(plan, u)
 
 
+@functools.lru_cache(maxsize=None)
 def _fused_size(n: int) -> bool:
     """Transform lengths of the fused propagation passes (2^a {1, 3, 5, 7} up to 4096, and 8192)."""
     return n == 8192 or bool(nat.lib().cx_fft_size_supported(int(n)))
@@ -238,6 +240,100 @@ def _cmul_planar(u, H, chromatic: bool):
     return launch(u.contiguous(), False)
 
 
+def _pair_key(v):
+    return v if type(v) is tuple else tuple(np.ravel(v).tolist())
+
+
+def _plan_key(field, zs, zshape, n, kykx, shift_yx, remove_evanescent, bandlimit, h_index):
+    dx = np.asarray(field.dx, dtype=np.float64)
+    return (type(field), dx.shape, dx.tobytes(), field.spectrum.wavelength.tobytes(), zs.tobytes(), tuple(zshape), float(n),
+            _pair_key(kykx), _pair_key(shift_yx), bool(remove_evanescent), bool(bandlimit),
+            None if h_index is None else np.asarray(h_index).tobytes())
+
+
+class _GeneralPlan:
+    """``_prop2d_general`` without gradients, prepared once per geometry: the
+    propagator's descriptor and planes, the four chirp-Z descriptors (y, x,
+    inverse y, inverse x) and their largest workspace."""
+
+    def __init__(self, field: Field, kernel, zs, zshape, n, pad, kykx, shift_yx, remove_evanescent, bandlimit, crop_w,
+                 prec):
+        from ..utils.czt import cx_czt_desc, workspace_bytes
+
+        ny, nx = field.spatial_shape
+        self.pad, self.crop = pad, crop_w
+        py, px = ny + 2 * pad[0], nx + 2 * pad[1]
+        W = field.n_wv
+        B = field.batch_shape
+        self.nb_in = int(np.prod(B)) if B else 1
+        self.out_batch = tuple(np.broadcast_shapes(B, zshape))
+        self.nb = int(np.prod(self.out_batch)) if self.out_batch else 1
+        self.spatial = (py, px) + ((W,) if field.chromatic else ())
+        self.pad_desc = nat.cx_ew_desc(n_batch=self.nb_in, ny=ny, nx=nx, n_wv=W, map_batched=0)
+        # one propagator per (z, wavelength); the field's batch shares it unless z runs over it
+        f_planes, h_batch, _, nb_h = _plan_planes(field, zs if zshape else zs[:1], zshape, py, px, shift_yx, bandlimit, prec,
+                                                  batch_shape=())
+        self.h_shape, self.h_planes = tuple(h_batch), nb_h
+        d = nat.cx_prop2d_desc()
+        d.ny, d.nx, d.n_wv, d.n_in_planes, d.n_out_planes = py, px, W, W, nb_h * W
+        d.kernel, d.precision = kernel, config.precision_code(prec)
+        d.remove_evanescent, d.bandlimit, d.n_medium = int(bool(remove_evanescent)), int(bool(bandlimit)), float(n)
+        ky0, kx0 = np.asarray(kykx, dtype=np.float64).reshape(2)
+        d.ky0, d.kx0 = float(ky0), float(kx0)
+        self.h_desc, self.planes = d, f_planes
+        self.mul_desc = nat.cx_ew_desc(n_batch=self.nb, ny=py, nx=px, n_wv=W, map_batched=-1 if nb_h == 1 else 1)
+        self.czt = []
+        for length, outer, inner, sign in ((py, self.nb, px * W, -1), (px, self.nb * py, W, -1), (py, self.nb, px * W, 1),
+                                           (px, self.nb * py, W, 1)):
+            c = cx_czt_desc()
+            c.n, c.m, c.L, c.inner, c.n_vec = length, length, 0, inner, outer * inner
+            c.in_ostride, c.in_istride, c.in_estride = length * inner, 1, inner
+            c.out_ostride, c.out_istride, c.out_estride = length * inner, 1, inner
+            w = complex(np.exp(sign * 2j * np.pi / length))
+            c.a_re, c.a_im, c.w_re, c.w_im = 1.0, 0.0, w.real, w.imag
+            c.mod_n, c.layout, c.scale = -1, 0 if inner == 1 else 1, 1.0 if sign < 0 else 1.0 / length
+            self.czt.append(c)
+        self.ws_bytes = max(workspace_bytes(c) for c in self.czt)
+
+    def run(self, field: Field):
+        from ..utils.czt import _lib
+
+        torch = nat.torch_mod()
+        L = _lib()
+        dev = field.device
+        st = nat.stream_handle(dev)
+        _, planes_dev = nat.device_table(self.h_desc, self.planes, dev, lambda d: 0)
+        u = field.u.to(torch.complex64).contiguous()
+        spatial, chrom = self.spatial, field.chromatic
+        if self.pad[0] or self.pad[1]:
+            up = torch.empty((self.nb_in,) + spatial, dtype=torch.complex64, device=dev)
+            nat.check(L.cx_pad(self.pad_desc, self.pad[0], self.pad[1], 0.0, 0.0, nat.ptr(u), nat.ptr(up), st))
+            u = up
+        if self.nb != self.nb_in:
+            u = u.reshape(tuple(field.batch_shape) + spatial).expand(self.out_batch + spatial).contiguous()
+        H = torch.empty((self.h_planes * self.spatial[2] if chrom else self.h_planes,) + spatial[:2],
+                        dtype=torch.complex64, device=dev)
+        nat.check(L.cx_fill_propagator(self.h_desc, nat.ptr(planes_dev), nat.ptr(H), st))
+        if self.h_planes > 1 and self.h_planes != self.nb:
+            W = self.spatial[2] if chrom else 1
+            H = H.reshape(self.h_shape + (W,) + spatial[:2]).expand(self.out_batch + (W,) + spatial[:2]).contiguous()
+        a, b = (torch.empty((self.nb,) + spatial, dtype=torch.complex64, device=dev) for _ in range(2))
+        ws = nat.workspace(self.ws_bytes, dev)
+        w = nat.ptr(ws)
+        pa, pb = nat.ptr(a), nat.ptr(b)
+        nat.check(L.cx_czt(self.czt[0], nat.ptr(u), pa, w, self.ws_bytes, st))
+        nat.check(L.cx_czt(self.czt[1], pa, pb, w, self.ws_bytes, st))
+        nat.check(L.cx_cmul_planar(self.mul_desc, pb, nat.ptr(H), 0, pa, st))
+        nat.check(L.cx_czt(self.czt[2], pa, pb, w, self.ws_bytes, st))
+        nat.check(L.cx_czt(self.czt[3], pb, pa, w, self.ws_bytes, st))
+        out = a.reshape(self.out_batch + spatial)
+        cy, cx = self.crop
+        if cy or cx:
+            s = 3 if chrom else 2
+            out = out.narrow(out.ndim - s, cy, spatial[0] - 2 * cy).narrow(out.ndim - s + 1, cx, spatial[1] - 2 * cx).contiguous()
+        return out
+
+
 def _prop2d_general(field: Field, kernel: int, zs, zshape, n, pad, kykx, shift_yx, remove_evanescent,
                     bandlimit, mode, crop_w, prec, H=None, h_index=None):
     """kernel_propagate's FFT branch (functional/propagation.py:391-394) on a
@@ -251,6 +347,18 @@ def _prop2d_general(field: Field, kernel: int, zs, zshape, n, pad, kykx, shift_y
 
     torch = nat.torch_mod()
     py_, px_ = pad
+    if H is None and not nat.wants_grad(field.u):
+        key = ("general", kernel, tuple(field.u.shape), field.n_wv, field.chromatic, pad, crop_w, prec) + _plan_key(
+            field, zs, zshape, n, kykx, shift_yx, remove_evanescent, bandlimit, None)
+        plan = _HOST_PLANS.get(key)
+        if plan is None:
+            plan = _HOST_PLANS[key] = _GeneralPlan(field, kernel, zs, zshape, n, pad, kykx, shift_yx, remove_evanescent,
+                                                   bandlimit, crop_w, prec)
+            if len(_HOST_PLANS) > _PLAN_CACHE_SIZE:
+                _HOST_PLANS.popitem(last=False)
+        else:
+            _HOST_PLANS.move_to_end(key)
+        return plan.run(field)
     f = pad_field(field, (py_, px_)) if (py_ or px_) else field
     py, px = f.spatial_shape
     W = f.n_wv
@@ -315,12 +423,8 @@ def _run_prop2d(field: Field, kernel: int, zs, zshape, n, pad_width, kykx=(0.0, 
         return _prop2d_general(field, kernel, zs, zshape, n, (py_, px_), kykx, shift_yx, remove_evanescent, bandlimit,
                                mode, crop_w, prec, H=H, h_index=h_index)
     W = field.n_wv
-    key = (kernel, tuple(field.u.shape), field.batch_shape, W, field.chromatic, py_, px_, crop, mode, prec,
-           np.asarray(field.dx_wv, dtype=np.float64).tobytes(),
-           np.asarray(field.spectrum.wavelength, dtype=np.float64).tobytes(),
-           np.asarray(zs, dtype=np.float64).tobytes(), tuple(zshape), float(n), tuple(np.ravel(kykx).tolist()),
-           tuple(np.ravel(shift_yx).tolist()), bool(remove_evanescent), bool(bandlimit),
-           None if h_index is None else np.asarray(h_index).tobytes())
+    key = (kernel, tuple(field.u.shape), W, field.chromatic, py_, px_, crop, mode, prec) + _plan_key(
+        field, zs, zshape, n, kykx, shift_yx, remove_evanescent, bandlimit, h_index)
     hit = _HOST_PLANS.get(key)
     if hit is not None:
         _HOST_PLANS.move_to_end(key)

@@ -8,6 +8,8 @@ processed in coalesced column tiles.  Chirp phases are evaluated in FP64
 
 from __future__ import annotations
 
+import functools
+
 import numpy as np
 
 from .. import _native as nat
@@ -41,14 +43,24 @@ def _lib():
     return L
 
 
+@functools.lru_cache(maxsize=256)
+def _ws_bytes(d_bytes: bytes) -> int:
+    ws_b = nat.c_size_t(0)
+    nat.check(_lib().cx_czt_workspace_size(cx_czt_desc.from_buffer_copy(d_bytes), ws_b))
+    return ws_b.value
+
+
+def workspace_bytes(d: cx_czt_desc) -> int:
+    return _ws_bytes(bytes(d))
+
+
 def _launch_czt(d: cx_czt_desc, x, oshape, out=None):
     torch = nat.torch_mod()
     y = out if out is not None else torch.empty(oshape, dtype=torch.complex64, device=x.device)
     L = _lib()
-    ws_b = nat.c_size_t(0)
-    nat.check(L.cx_czt_workspace_size(d, ws_b))
-    ws = nat.workspace(ws_b.value, x.device)
-    nat.check(L.cx_czt(d, nat.ptr(x), nat.ptr(y), nat.ptr(ws), ws_b.value, nat.stream_handle(x.device)))
+    n_ws = workspace_bytes(d)
+    ws = nat.workspace(n_ws, x.device)
+    nat.check(L.cx_czt(d, nat.ptr(x), nat.ptr(y), nat.ptr(ws), n_ws, nat.stream_handle(x.device)))
     return y
 
 
