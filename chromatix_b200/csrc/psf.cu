@@ -2,6 +2,7 @@
 #include <cmath>
 #include <cstdlib>
 
+#include "pair_fft.cuh"
 #include "psf.cuh"
 
 namespace cx {
@@ -347,6 +348,17 @@ static cx_status psf_setup(const cx_psf_desc* d, const cx_psf_spectrum* spec, co
   a.CX = reinterpret_cast<float2*>(static_cast<char*>(workspace) + 256 + psf_t_bytes(d) + psf_m_bytes(d));
   a.CY = a.CX + psf_cx_bytes(d) / sizeof(float2);
   a.ldT = psf_ld(d);
+  // Both passes on pairs: T by tiles of 8 columns, so that the column pass
+  // reads contiguous memory and a row pair writes whole 128-byte lines.  By row
+  // the column pass fetches 32 bytes per row pitch, half of what the DRAM
+  // moves.  us per stack, 64 x 3 x 1280^2 and 128 x 1536^2 (both passes):
+  // by row 1530 / 2127; tiles of 4 columns 1383 / 2175, 8: 1397 / 1972,
+  // 16: 1468 / 2063, 64: 1476 / 2074.
+  // (A length with a pair plan is a multiple of 8; the other row and column
+  // passes know T by row only.)
+  const bool tiled = d->precision == CX_PREC_ACCURATE && pair_length(d->nx) && pair_length(d->ny);
+  a.shT = tiled ? 3 : 30;
+  a.rT = tiled ? 8 : a.ldT;
   // z planes per chunk: as many compact planes as the row-spectrum region holds
   const size_t zbytes = sizeof(float2) * (size_t)a.rowsum * a.ldT;
   int zc = (int)(psf_t_bytes(d) / zbytes);

@@ -55,9 +55,12 @@ struct PsfArgs {
   // CY (nz, rowsum), by stored row: exp(i qz (y dy - off_y)^2) (pair passes)
   float2* CY;
   int ldT;  // row pitch of T: nx, rounded up to even
+  // Element (r, k) of one wavelength's rows of T at (k >> shT) * (nrows << shT) + r * rT + (k & ((1 << shT) - 1)):
+  // by row (shT = 30, rT = ldT), or by tile of 1 << shT = rT = 8 columns
+  int shT, rT;
   const double* z;
   const float* phase;
-  float2* T;  // (zc, rowsum, ldT): only the rows [ylo_w, ylo_w + nrows_w) of each wavelength
+  float2* T;  // rowsum * ldT elements per plane: only the rows [ylo_w, ylo_w + nrows_w) of each wavelength
   const unsigned long long* counts;  // [0, 8): pupil pixel counts per wavelength
   const int* srange;                 // [0, 8): ny - first support row ; [8, 16): last support row + 1
   float* out;

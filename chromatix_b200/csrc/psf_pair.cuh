@@ -48,7 +48,8 @@ __global__ void __launch_bounds__(PsfPairRows<NX>::THREADS, PsfPairRows<NX>::MIN
     const float2* cyz = a.CY + (size_t)(a.z0 + zl) * a.rowsum + a.prefix[w] + r;
     const c2 cy = ppack(cyz[0], cyz[two ? 1 : 0]);
     const int xlo = a.xlo[w], nc = a.ncols[w];
-    float2* dst = a.T + ((size_t)zl * a.rowsum + a.prefix[w] + r) * a.ldT;
+    float2* dst = a.T + ((size_t)zl * a.rowsum + a.prefix[w]) * a.ldT + (size_t)r * a.rT;
+    const int sh = a.shT, tile = a.nrows[w] << (sh & 15), low = (1 << sh) - 1, rT = a.rT;
     auto load = [&](int n) -> c2 {
       const int c = add_mod(n, NX / 2, NX) - xlo;  // ifftshift along x, then the box column
       const bool ok = (unsigned)c < (unsigned)nc;
@@ -56,8 +57,9 @@ __global__ void __launch_bounds__(PsfPairRows<NX>::THREADS, PsfPairRows<NX>::MIN
     };
     auto out = [&](int k, c2 v) {
       if (valid) {
-        dst[k] = pfirst(v);
-        if (two) dst[a.ldT + k] = psecond(v);
+        float2* p = dst + (k >> sh) * tile + (k & low);
+        p[0] = pfirst(v);
+        if (two) p[rT] = psecond(v);
       }
     };
     sync();  // the pair's previous transform has been read
@@ -71,8 +73,8 @@ __global__ void __launch_bounds__(PsfPairRows<NX>::THREADS, PsfPairRows<NX>::MIN
 // wavelength's sum stored fftshifted
 // --------------------------------------------------------------------------
 // V = 2 VP columns: the widest tile of at most 256 lanes that leaves room for
-// three CTAs per SM, at least 4 columns (32-byte row segments, whole sectors
-// of the L2-resident row spectra): 4 columns at 1280, 8 at 768, 16 at 256.
+// three CTAs per SM, at least 4 columns (32-byte row segments, whole sectors):
+// 4 columns at 1280, 8 at 768, 16 at 256.
 template <int NY>
 struct PsfPairCols {
   static constexpr int L = PairPlan<NY>::L;
@@ -109,6 +111,7 @@ __global__ void __launch_bounds__(PsfPairCols<NY>::THREADS, PsfPairCols<NY>::MIN
   auto sync = [] { __syncthreads(); };
   const int tiles_x = (a.nx + V - 1) / V;
   const long total = (long)tiles_x * a.zc;
+  const int rT = a.rT;
   for (long i = blockIdx.x; i < total; i += gridDim.x) {
     const int zl = (int)(i / tiles_x);
     const int x = (int)(i % tiles_x) * V + 2 * c;
@@ -118,10 +121,11 @@ __global__ void __launch_bounds__(PsfPairCols<NY>::THREADS, PsfPairCols<NY>::MIN
     for (int w = 0; w < a.W; ++w) {
       const float dens = (float)a.wv[w].dens;
       const int slo = support_lo(a, w), shi = support_hi(a, w);
-      const float2* src = a.T + ((size_t)zl * a.rowsum + a.prefix[w] - a.ylo[w]) * a.ldT + x;
+      const float2* src = a.T + ((size_t)zl * a.rowsum + a.prefix[w]) * a.ldT - (ptrdiff_t)a.ylo[w] * a.rT +
+                          (size_t)(x >> a.shT) * ((size_t)a.nrows[w] << (a.shT & 15)) + (x & ((1 << a.shT) - 1));
       auto load = [&](int n) -> c2 {
         const int y = add_mod(n, NY / 2, NY);  // ifftshift along y
-        return ppack(ld4z(src + (size_t)y * a.ldT, ok && y >= slo && y < shi));
+        return ppack(ld4z(src + (size_t)y * rT, ok && y >= slo && y < shi));
       };
       const bool first = w == 0, last = w + 1 == a.W;
       auto out = [&](int k, c2 v) {
