@@ -36,7 +36,9 @@ struct ConvPairRows {
   static constexpr int TWB = (F::TW * (int)sizeof(float2) + 15) & ~15;
   static constexpr size_t SMEM = TWB + sizeof(float4) * (size_t)ROWS * F::ELEMS;
   static constexpr int WARPS = (THREADS + 31) / 32;
-  static constexpr int MINB = 16 / WARPS > 0 ? 16 / WARPS : 1;
+  // 20 warps per SM: the pass waits on loads and barriers.  16 -> 20: 1243 -> 1114 us at M = 1536 (64 planes; two
+  // CTAs -> three), 794 -> 752 at 1280, 449 -> 443 at 1024; one-warp CTAs only lose registers (256: 28 -> 30)
+  static constexpr int MINB = WARPS == 1 ? 16 : (20 / WARPS > 0 ? 20 / WARPS : 1);
 };
 
 template <int M>
@@ -112,16 +114,21 @@ __global__ void __launch_bounds__(ConvPairRows<M>::THREADS, ConvPairRows<M>::MIN
 // --------------------------------------------------------------------------
 // Work units (column, plane) split in equal contiguous ranges over the
 // resident CTAs (no last wave); a range's sums go to St when it leaves a column.
+// The first stage's twiddles stay in registers: 6 KB less shared memory let a
+// third CTA per SM in at 3072 (64 planes: 1347 -> 1284 us; 4096: 2404 -> 2271;
+// 512 to 2560: within 3 %).
 template <int P>
 struct ConvPairCols {
   using F = PairFFT<P, 1>;
   static constexpr int L = F::L;
   static constexpr int THREADS = L;
-  static constexpr int TWB = (F::TW * (int)sizeof(float2) + 15) & ~15;
+  static constexpr int TWB = ((F::TW - F::T2) * (int)sizeof(float2) + 15) & ~15;
   static constexpr size_t ACC_OFF = TWB + sizeof(float4) * (size_t)F::ELEMS;
   static constexpr size_t SMEM = ACC_OFF + sizeof(float2) * (size_t)P;
   static constexpr int WARPS = (THREADS + 31) / 32;
-  static constexpr int MINB = 18 / WARPS > 0 ? 18 / WARPS : 1;
+  // up to 20 warps per SM, as far as their shared memory goes
+  static constexpr int FIT = (int)(227 * 1024 / (SMEM + 1024));
+  static constexpr int MINB = 20 / WARPS < 1 || FIT < 1 ? 1 : (20 / WARPS < FIT ? 20 / WARPS : FIT);
   static_assert(SMEM <= 227 * 1024, "convolution column does not fit one CTA");
 };
 
@@ -133,8 +140,10 @@ __global__ void __launch_bounds__(ConvPairCols<P>::THREADS, ConvPairCols<P>::MIN
   float2* tw = reinterpret_cast<float2*>(smem);
   float4* s = reinterpret_cast<float4*>(smem + C::TWB);
   float2* acc = reinterpret_cast<float2*>(smem + C::ACC_OFF);
-  F::load_tables(tw, a.twg, threadIdx.x, blockDim.x);
+  F::template load_tables<F::T2>(tw, a.twg, threadIdx.x, blockDim.x);
+  tw -= F::T2;
   const int t = threadIdx.x;
+  const typename F::Powers w1 = F::first_powers(a.twg, t);
   auto sync = [] { __syncthreads(); };
   const float4* T = reinterpret_cast<const float4*>(a.T);
   const long units = (long)a.NC * a.zc;
@@ -160,7 +169,9 @@ __global__ void __launch_bounds__(ConvPairCols<P>::THREADS, ConvPairCols<P>::MIN
     };
     __syncthreads();  // the previous column has been read
     // rows >= HB are zero and P >= 2 HB
-    F::template transform<false, pair_lower_mask<P>()>(s, tw, t, load, out, sync);
+    F::template first<false, pair_lower_mask<P>()>(s, w1, t, load);
+    F::template inner<false>(s, tw, t, sync);
+    F::template last<false>(s, t, out);
     fresh = leave;
   }
 }

@@ -380,14 +380,16 @@ struct PairFFT {
   static constexpr int T2 = ptw_powers(R1) * M, T3 = T2 + (S > 2 ? ptw_powers(R2) * M2 : 0);
   static constexpr int TW = T3 + (S > 3 ? ptw_powers(R3) * M3 : 0);
 
-  // fill the tables from the length's table w_N^m (m < N) in global memory
+  // fill the tables from the length's table w_N^m (m < N) in global memory; FROM = T2: all but the first stage's
+  // (a kernel that keeps its lanes' first-stage powers in registers passes `tw` - T2 from there on)
+  template <int FROM = 0>
   __device__ static void load_tables(float2* tw, const float2* __restrict__ twg, int tid, int nthreads) {
     const float2* g = twg + tw_offset(N);
-    for (int i = tid; i < TW; i += nthreads) {
+    for (int i = FROM + tid; i < TW; i += nthreads) {
       const int base = i < T2 ? 0 : (i < T3 ? T2 : T3), block = i < T2 ? M : (i < T3 ? M2 : M3);
       const int step = i < T2 ? 1 : (i < T3 ? R1 : R1 * R2);
       const int j = (i - base) % block, pw = (i - base) / block;
-      tw[i] = g[((j * step) << pw) % N];
+      tw[i - FROM] = g[((j * step) << pw) % N];
     }
   }
 
@@ -411,6 +413,29 @@ struct PairFFT {
 #pragma unroll
       for (int q = 0; q < R1; ++q) sstore(s + (q * PITCH + j) * VP, v[q]);
     });
+  }
+  // A lane's first butterfly is always its t-th: its powers can stay in
+  // registers over all of a kernel's transforms, 8 registers for a quarter of
+  // the first stage's shared-memory reads and the largest table.
+  struct Powers {
+    float2 w[ptw_powers(R1)];
+  };
+  __device__ __forceinline__ static Powers first_powers(const float2* __restrict__ twg, int t) {
+    Powers p;
+#pragma unroll
+    for (int i = 0; i < ptw_powers(R1); ++i) p.w[i] = twg[tw_offset(N) + ((t << i) % N)];
+    return p;
+  }
+  template <bool INV, unsigned ZM = 0u, class Load>
+  __device__ __forceinline__ static void first(float4* s, const Powers& w, int t, Load& load) {
+    static_assert(M == L, "one first-stage butterfly per lane");
+    c2 v[R1];
+#pragma unroll
+    for (int r = 0; r < R1; ++r) v[r] = ((ZM >> r) & 1u) ? pzero() : load(t + r * M);
+    PDFT<R1, INV>::run(v);
+    ptwiddle<R1, INV, 1>(v, w.w);
+#pragma unroll
+    for (int q = 0; q < R1; ++q) sstore(s + (q * PITCH + t) * VP, v[q]);
   }
   // the inner stages (2 of three; 2 and 3 of four)
   template <bool INV, bool BACK>
