@@ -1,4 +1,5 @@
 // C API of the Fourier-multiplier propagation (kernels in prop2d.cuh).
+#include "pair_fft.cuh"
 #include "prop2d.cuh"
 
 namespace cx {
@@ -16,6 +17,9 @@ __global__ void k_fill_propagator(float2* __restrict__ H, Prop2DArgs a) {
   }
 }
 
+
+static size_t ws_T_bytes(const Prop2DArgs& a) { return sizeof(float2) * (size_t)a.n_in_planes * a.ny * a.px; }
+static size_t ws_T2_bytes(const Prop2DArgs& a) { return sizeof(float2) * (size_t)a.n_out_planes * a.out_ny * a.px; }
 
 static cx_status make_args(const cx_prop2d_desc* d, Prop2DArgs* a) {
   if (!d) {
@@ -81,11 +85,21 @@ static cx_status make_args(const cx_prop2d_desc* d, Prop2DArgs* a) {
     set_error("padded grid %dx%d: FFT length not supported", a->py, a->px);
     return CX_ERR_UNSUPPORTED;
   }
+  // All passes on pairs: spectra by tiles of 8 columns, so that the column pass
+  // reads and writes contiguous memory (by row it moves 16 to 64 bytes per row
+  // pitch) and a row pair still fills 128-byte lines.  us of the three passes,
+  // 64 x 512^2 -> 1024^2 and one 4096^2 -> 8192^2: by row 651 / 1217; tiles of
+  // 2 columns 733 / 1099, 4: 637 / 1052, 8: 617 / 1064, 16: 632 / 1172.
+  // Up to half of the L2 (64 MiB of both spectra) the row order costs the column
+  // pass nothing and the tiles cost the row pass its wide stores: 3 x 600 x 800
+  // 124 us by row, 127 by tile; 8 x 640^2 -> 1024^2 (84 MB) 191 and 185.
+  // (A length with a pair plan is a multiple of 8.)
+  if (a->precision != CX_PREC_SPLIT16 && pair_length(a->py) && pair_length(a->px) &&
+      ws_T_bytes(*a) + ws_T2_bytes(*a) > ((size_t)64 << 20))
+    a->tsh = 3;
   return CX_OK;
 }
 
-static size_t ws_T_bytes(const Prop2DArgs& a) { return sizeof(float2) * (size_t)a.n_in_planes * a.ny * a.px; }
-static size_t ws_T2_bytes(const Prop2DArgs& a) { return sizeof(float2) * (size_t)a.n_out_planes * a.out_ny * a.px; }
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 }  // namespace cx

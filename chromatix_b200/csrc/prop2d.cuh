@@ -27,6 +27,9 @@ struct Prop2DArgs {
   int precise;   // 1: FP64 sin/cos (tables reused many times); 0: FP64 reduction + hardware sin/cos
   int conj_h;    // 1: use conj(H) (adjoint passes; any kernel kind)
   int pdl = 0;   // 1: the table column pass may start beside its predecessor (H complete before that one's)
+  // Stored spectra by row (30), or by tiles of 1 << tsh columns (pair passes only): a tile's rows are contiguous,
+  // element (r, k) of a plane of n rows at (k >> tsh) * (n << tsh) + (r << tsh) + (k & ((1 << tsh) - 1))
+  int tsh = 30;
   const cx_plane* planes;
   const float2* H;
   const float2* twg;  // device twiddle tables (ensure_twiddles)

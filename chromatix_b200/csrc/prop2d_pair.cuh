@@ -24,6 +24,9 @@ constexpr unsigned pair_band_mask() {
   return m;
 }
 
+// row pitch of the stored spectra
+__device__ __forceinline__ int prop_pitch(const Prop2DArgs& a) { return a.tsh == 30 ? a.px : 1 << a.tsh; }
+
 // --------------------------------------------------------------------------
 // pass A: forward row transform of row pairs, zero padding in the loader
 // --------------------------------------------------------------------------
@@ -43,6 +46,7 @@ __global__ void __launch_bounds__(PairRows<NX>::THREADS, PairRows<NX>::MINB)
   const int npair = (a.ny + 1) / 2;
   const long total = (long)(a.n_in_planes / a.W) * npair * a.W;
   const bool band = 4 * a.pad_x >= NX && 4 * (a.pad_x + a.nx) <= 3 * NX;
+  const int low = (1 << a.tsh) - 1, rT = prop_pitch(a), tstep = a.ny * rT;
   __syncthreads();
   for (long base = (long)blockIdx.x * C::TEAMS; base < total; base += (long)gridDim.x * C::TEAMS) {
     const long item = base + team;
@@ -54,7 +58,7 @@ __global__ void __launch_bounds__(PairRows<NX>::THREADS, PairRows<NX>::MINB)
     const float2* ub = a.in_ptrs ? a.in_ptrs[b] : u + (size_t)b * a.ny * a.nx * a.W;
     const float2* src = ub + (size_t)y * a.nx * a.W + w;
     const size_t up = two ? (size_t)a.nx * a.W : 0;
-    float2* dst = T + ((size_t)(b * a.W + w) * a.ny + y) * a.px;
+    float2* dst = T + (size_t)(b * a.W + w) * a.ny * a.px + (size_t)y * rT;
     auto load = [&](int n) -> c2 {
       const int x = n - a.pad_x;
       if (!valid || (unsigned)x >= (unsigned)a.nx) return pzero();
@@ -62,8 +66,9 @@ __global__ void __launch_bounds__(PairRows<NX>::THREADS, PairRows<NX>::MINB)
       return ppack(p[0], p[up]);
     };
     auto out = [&](int k, c2 v) {
-      if (valid) dst[k] = pfirst(v);
-      if (two) dst[a.px + k] = psecond(v);
+      float2* p = dst + (k >> a.tsh) * tstep + (k & low);
+      if (valid) p[0] = pfirst(v);
+      if (two) p[rT] = psecond(v);
     };
     sync();  // the pair's previous transform has been read
     if (band)
@@ -89,6 +94,7 @@ __global__ void __launch_bounds__(PairRows<NX>::THREADS, PairRows<NX>::MINB)
   auto sync = [&] { C::sync(team); };
   const int npair = (a.out_ny + 1) / 2;
   const long total = (long)(a.n_out_planes / a.W) * npair * a.W;
+  const int low = (1 << a.tsh) - 1, rT = prop_pitch(a), tstep = a.out_ny * rT;
   __syncthreads();
   for (long base = (long)blockIdx.x * C::TEAMS; base < total; base += (long)gridDim.x * C::TEAMS) {
     const long item = base + team;
@@ -97,13 +103,14 @@ __global__ void __launch_bounds__(PairRows<NX>::THREADS, PairRows<NX>::MINB)
     const long bi = valid ? item / a.W : 0;
     const int b = (int)(bi / npair), r = 2 * (int)(bi % npair);
     const bool two = valid && r + 1 < a.out_ny;
-    const float2* src = T2 + ((size_t)(b * a.W + w) * a.out_ny + r) * a.px;
-    const size_t up = two ? (size_t)a.px : 0;
+    const float2* src = T2 + (size_t)(b * a.W + w) * a.out_ny * a.px + (size_t)r * rT;
+    const int up = two ? rT : 0;
     float2* ob = a.out_ptrs ? a.out_ptrs[b] : outp + (size_t)b * a.out_ny * a.out_nx * a.W;
     float2* dst = ob + (size_t)r * a.out_nx * a.W + w;
     auto load = [&](int n) -> c2 {
       if (!valid) return pzero();
-      return ppack(src[n], src[up + n]);
+      const float2* p = src + (n >> a.tsh) * tstep + (n & low);
+      return ppack(p[0], p[up]);
     };
     auto out = [&](int k, c2 v) {
       const int x = k - a.out_x0;
@@ -178,7 +185,7 @@ __global__ void __launch_bounds__(PropPairCols<NY, TABLE>::THREADS, PropPairCols
   const int c = threadIdx.x % VP, t = threadIdx.x / VP;
   float4* s = s0 + c;
   auto sync = [] { __syncthreads(); };
-  const int tiles_x = (a.px + V - 1) / V;
+  const int tiles_x = (a.px + V - 1) / V, rT = prop_pitch(a);
   const float scale = 1.0f / ((float)a.py * (float)a.px);
   const bool band = 4 * a.pad_y >= NY && 4 * (a.pad_y + a.ny) <= 3 * NY;
   // CTAs of adjacent column tiles run at the same time (their 32- or 64-byte row segments share DRAM pages); a
@@ -194,11 +201,12 @@ __global__ void __launch_bounds__(PropPairCols<NY, TABLE>::THREADS, PropPairCols
     const cx_plane& pl = a.planes[q];
     const int x = x0 + 2 * c;
     const bool ok0 = x < a.px, ok1 = x + 1 < a.px;
-    const float2* src = T + (size_t)pl.in_plane * a.ny * a.px + x;
+    const int xt = x >> a.tsh, xl = x & ((1 << a.tsh) - 1);
+    const float2* src = T + (size_t)pl.in_plane * a.ny * a.px + (size_t)(xt * rT) * a.ny + xl;
     auto load = [&](int n) -> c2 {
       const int r = n - a.pad_y;
       const bool ok = ok0 && (unsigned)r < (unsigned)a.ny;
-      const float2* p = src + (ptrdiff_t)r * a.px;
+      const float2* p = src + (ptrdiff_t)r * rT;
       if constexpr (VEC) return ppack(ld4z(p, ok));
       return ppack(ld2z(p, ok), ld2z(p + 1, ok && ok1));
     };
@@ -303,12 +311,12 @@ __global__ void __launch_bounds__(PropPairCols<NY, TABLE>::THREADS, PropPairCols
         F::template centre<false>(s, t, f, even ? 0 : half * HB, even || half ? NB : HB);
       }
     }
-    float2* dst = T2 + (size_t)q * a.out_ny * a.px + x;
+    float2* dst = T2 + (size_t)q * a.out_ny * a.px + (size_t)(xt * rT) * a.out_ny + xl;
     auto out = [&](int n, c2 v) {
       const int r = n - a.out_y0;
       if (!ok0 || (unsigned)r >= (unsigned)a.out_ny) return;
       v = pscale(v, scale);
-      float2* p = dst + (size_t)r * a.px;
+      float2* p = dst + (size_t)r * rT;
       if constexpr (VEC) {
         *reinterpret_cast<float4*>(p) = punpack(v);
       } else {

@@ -227,3 +227,29 @@ def test_mbs_strided_passes(n, axis):
     source.field = to_cuda(src)
     E = mbs.solve(sample, source, maxiter=1, tol=0.0, shift=op.bias, scale=op.scale).cpu().numpy()
     assert O.rel_l2(E, op.step(op.prec_y) * op.num_scale) < 2 * BAR
+
+
+@pytest.mark.parametrize("ny,nx,pad,batch", [(2048, 2560, (0, 0), 1), (2048, 2560, (256, 0), 1), (640, 896, (0, 0), 10),
+                                             (4096, 640, (0, 0), 2)])
+def test_spectra_by_tile(ny, nx, pad, batch):
+    """Spectra too large for half of the L2 are stored by tiles of eight columns: against the same field in batches
+    that are stored by row, bit by bit (the arithmetic is the same)."""
+    import torch
+
+    import chromatix_b200.functional as cf
+
+    rng = np.random.default_rng(ny + nx)
+    u = _crand(rng, (batch, ny, nx))
+    H = _crand(rng, (ny, nx))
+    f = _field(u)
+    big = cf.transfer_propagate(f, 30.0, 1.33, pad, mode="same").u
+    if batch > 2:
+        small = [cf.transfer_propagate(_field(u[b:b + 1]), 30.0, 1.33, pad, mode="same").u for b in range(batch)]
+        assert torch.equal(big, torch.cat(small))
+    ref = np.fft.ifft2(np.fft.fft2(u.astype(np.complex128)) * H)
+    assert O.rel_l2(cf.kernel_propagate(f, to_cuda(H)).u.cpu().numpy(), ref) < BAR
+    fy, fx = np.fft.fftfreq(ny + 2 * pad[0], 0.3), np.fft.fftfreq(nx + 2 * pad[1], 0.3)
+    P = np.exp(-1j * np.pi * 0.532 * 30.0 / 1.33 * (fy[:, None] ** 2 + fx[None, :] ** 2))
+    v = np.pad(u.astype(np.complex128), [(0, 0), (pad[0], pad[0]), (pad[1], pad[1])])
+    out = np.fft.ifft2(np.fft.fft2(v) * P)[:, pad[0]:pad[0] + ny, pad[1]:pad[1] + nx]
+    assert O.rel_l2(big.cpu().numpy(), out) < BAR
