@@ -297,7 +297,7 @@ def gpu_arm(args):
                                                             / (ms_e2e * 1e-3) / 1e9, 1)},
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
                          "frac": round(achieved / hbm, 4), "traffic": traffic if best == "accurate" else None,
-                         "kernel": ("k_psf_cols<1280> (column FFT + spectral intensity)" if best == "accurate" else
+                         "kernel": ("k_psf_cols_pair<1280> (column FFT + spectral intensity)" if best == "accurate" else
                                     "k_psf_cols_tc<40,32> (tensor-core column FFT + spectral intensity)"),
                          "kernel_ms": round(kern["ms"], 5), "peak_source": peak_src},
             "transform_form": best,

@@ -46,10 +46,6 @@ void set_error(const char* fmt, ...);
 #define CX_FOR_EACH_CZT_LONG_SIZE(X) X(4608) X(5120) X(6144) X(7168)
 #define CX_FOR_EACH_LONG_SIZE(X) CX_FOR_EACH_CZT_LONG_SIZE(X) X(8192)
 #define CX_FOR_EACH_1D_SIZE(X) CX_FOR_EACH_SIZE(X) CX_FOR_EACH_LONG_SIZE(X)
-// The Fourier-multiplier propagation passes also take 8192 (a 4096^2 field
-// padded by 2048 per side, the reference's high-resolution band-limited ASM
-// example); a 8192-point row or column is one team of 512 lanes per CTA.
-#define CX_FOR_EACH_PROP_SIZE(X) CX_FOR_EACH_SIZE(X) X(8192)
 
 inline bool size_supported(int n) {
   switch (n) {
