@@ -253,3 +253,61 @@ def test_spectra_by_tile(ny, nx, pad, batch):
     v = np.pad(u.astype(np.complex128), [(0, 0), (pad[0], pad[0]), (pad[1], pad[1])])
     out = np.fft.ifft2(np.fft.fft2(v) * P)[:, pad[0]:pad[0] + ny, pad[1]:pad[1] + nx]
     assert O.rel_l2(big.cpu().numpy(), out) < BAR
+
+
+@pytest.mark.parametrize("n,m", [(64, 65), (65, 64), (100, 61), (129, 96), (300, 213), (513, 512), (700, 1349),
+                                 (2000, 561), (2047, 2050), (4096, 4096)])
+def test_chirp_z_pairs(n, m):
+    """n + m - 1 at and beside a transform length, along contiguous rows (an odd number of them: half a pair) and along
+    strided columns (odd and even numbers, a ragged last tile), against the sums in FP64.  Three FP32 transforms, three
+    factors in 32 bits and the filter's spectrum: within the propagation's tolerance."""
+    from chromatix_b200.utils.czt import czt
+
+    rng = np.random.default_rng(n + m)
+    a, w = np.exp(0.21j), np.exp(-1.7j / max(n, m))
+    j, k = np.arange(n), np.arange(m)
+    D = np.exp(1j * (np.angle(w) * np.outer(k, j) - np.angle(a) * j))
+    for shape, axis in (((3, n), -1), ((2, n, 5), 1), ((n, 18), 0)):
+        x = _crand(rng, shape)
+        out = czt(to_cuda(x), m, a, w, axis=axis).cpu().numpy()
+        ref = np.moveaxis(np.moveaxis(x.astype(np.complex128), axis, -1) @ D.T, -1, axis)
+        assert O.rel_l2(out, ref) < BAR, shape
+
+
+@pytest.mark.parametrize("batch,ny,nx,wv", [(1, 5, 7, 1), (3, 6, 10, 1), (4, 33, 31, 2), (17, 64, 64, 3)])
+def test_phase_factor_over_a_batch(batch, ny, nx, wv):
+    """One phase map for every field of a batch and one map per field, one and several wavelengths, odd and even row
+    lengths.  FP32 sin / cos of arguments below 2 pi and one product: 4e-7."""
+    import chromatix_b200.functional as cf
+
+    rng = np.random.default_rng(batch + nx)
+    lam = np.array([0.5, 0.45, 0.6][:wv]) if wv > 1 else 0.5
+    u = _crand(rng, (batch, ny, nx) + ((wv,) if wv > 1 else ()))
+    for shape in ((ny, nx), (batch, ny, nx)):
+        ph = rng.uniform(-3, 3, shape).astype(np.float32)
+        f = _field(u, lam=lam)
+        out = cf.phase_change(f, to_cuda(ph)).u.cpu().numpy()
+        p = ph.astype(np.float64)
+        if wv > 1:
+            p = p[..., None] * f.spectrum.spectral_modulation
+        assert O.rel_l2(out, u * np.exp(1j * p)) < 4e-7
+
+
+@pytest.mark.parametrize("shape", [(45, 75), (81, 99)])
+def test_lengths_without_a_pass(shape):
+    """Padded lengths with no fused pass: the planned route (no gradient asked for) against the route through autograd
+    and against FP64; chirp-Z transforms instead of FFTs, twice the propagation's tolerance."""
+    import torch
+
+    import chromatix_b200.functional as cf
+
+    rng = np.random.default_rng(shape[0])
+    u = _crand(rng, (2,) + shape)
+    f, g = _field(u), _field(u)
+    g.u.requires_grad_(True)
+    out = cf.asm_propagate(f, 25.0, 1.33, 6, mode="same").u
+    grad = cf.asm_propagate(g, 25.0, 1.33, 6, mode="same").u.detach()
+    assert torch.allclose(out, grad, rtol=0, atol=1e-5 * float(grad.abs().max()))
+    for b in range(2):
+        ref = O.asm_propagate(O.field_build(u[b], 0.3, 0.532), 25.0, 1.33, 6, mode="same").u
+        assert O.rel_l2(out[b].cpu().numpy(), np.asarray(ref).reshape(shape)) < 2 * BAR
