@@ -240,15 +240,23 @@ def _cmul_planar(u, H, chromatic: bool):
     return launch(u.contiguous(), False)
 
 
+_PLAIN = (float, int)
+
+
 def _pair_key(v):
-    return v if type(v) is tuple else tuple(np.ravel(v).tolist())
+    """The values of a (y, x) pair: a tuple of Python numbers as it is (their
+    conversion costs as much as the rest of the key), any other form (arrays,
+    tensors, tuples of them) converted, since those hash by identity or not at all."""
+    if type(v) is tuple and len(v) == 2 and type(v[0]) in _PLAIN and type(v[1]) in _PLAIN:
+        return v
+    return tuple(np.asarray(v, dtype=np.float64).ravel().tolist())
 
 
 def _plan_key(field, zs, zshape, n, kykx, shift_yx, remove_evanescent, bandlimit, h_index):
     dx = np.asarray(field.dx, dtype=np.float64)
-    return (type(field), dx.shape, dx.tobytes(), field.spectrum.wavelength.tobytes(), zs.tobytes(), tuple(zshape), float(n),
-            _pair_key(kykx), _pair_key(shift_yx), bool(remove_evanescent), bool(bandlimit),
-            None if h_index is None else np.asarray(h_index).tobytes())
+    return (type(field), dx.shape, dx.tobytes(), np.asarray(field.spectrum.wavelength, dtype=np.float64).tobytes(),
+            np.asarray(zs, dtype=np.float64).tobytes(), tuple(zshape), float(n), _pair_key(kykx), _pair_key(shift_yx),
+            bool(remove_evanescent), bool(bandlimit), None if h_index is None else np.asarray(h_index).tobytes())
 
 
 class _GeneralPlan:
