@@ -163,8 +163,17 @@ _OPT_PLANS = collections.OrderedDict()
 _OPT_PLANS_SIZE = 64
 
 
-def _host_bytes(v):
-    return None if v is None else np.asarray(v).tobytes()
+def _host_key(v, dtype=np.float64):
+    """Shape and values of a number or an array of them."""
+    if v is None:
+        return None
+    v = np.asarray(v, dtype=dtype)
+    return v.shape, v.tobytes()
+
+
+def _number(v) -> float:
+    """A number given as a scalar or as an array of one element."""
+    return float(v) if np.ndim(v) == 0 else float(np.asarray(v, dtype=np.float64).reshape(()))
 
 
 def run_optfft(field: Field, z: float, n: float, pad_width=(0, 0), crop_width=(0, 0), post=1.0 + 0j,
@@ -174,9 +183,11 @@ def run_optfft(field: Field, z: float, n: float, pad_width=(0, 0), crop_width=(0
     prec = precision or config.get_precision()
     py_, px_ = pad_width
     cy, cx = crop_width
-    key = (type(field), tuple(field.u.shape), np.shape(field.dx), _host_bytes(field.dx), np.shape(field.origin),
-           _host_bytes(field.origin), _host_bytes(field.spectrum.wavelength), z, n, py_, px_, cy, cx,
-           np.shape(post), _host_bytes(post), _host_bytes(chirp_in), _host_bytes(chirp_out), pupil_D, prec)
+    z, n = _number(z), _number(n)
+    pupil_D = None if pupil_D is None else _number(pupil_D)
+    key = (type(field), tuple(field.u.shape), _host_key(field.dx), _host_key(field.origin),
+           _host_key(field.spectrum.wavelength), z, n, py_, px_, cy, cx, _host_key(post, np.complex128),
+           _host_key(chirp_in), _host_key(chirp_out), pupil_D, prec)
     hit = _OPT_PLANS.get(key)
     if hit is not None:
         _OPT_PLANS.move_to_end(key)
