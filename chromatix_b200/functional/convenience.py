@@ -9,6 +9,7 @@ the store.
 from __future__ import annotations
 
 import collections
+import operator
 
 import numpy as np
 
@@ -181,8 +182,7 @@ def run_optfft(field: Field, z: float, n: float, pad_width=(0, 0), crop_width=(0
     """Launch the chirped optical FFT; returns (u_out, du (wv, 2))."""
     nat.require_cuda(field.u, "Field.u")
     prec = precision or config.get_precision()
-    py_, px_ = pad_width
-    cy, cx = crop_width
+    (py_, px_), (cy, cx) = map(operator.index, pad_width), map(operator.index, crop_width)
     z, n = _number(z), _number(n)
     pupil_D = None if pupil_D is None else _number(pupil_D)
     key = (type(field), tuple(field.u.shape), _host_key(field.dx), _host_key(field.origin),

@@ -76,3 +76,16 @@ def test_factors_by_value_not_by_bytes(planes):
     for chirp in (one, one.view(np.int64)):
         C.run_optfft(f, 100.0, 1.0, chirp_in=chirp)
         np.testing.assert_array_equal(planes[-1]["chirp_in"], chirp.astype(np.float64))
+
+
+@pytest.mark.parametrize("make", [lambda: torch.tensor(2), lambda: np.array(2)])
+def test_padding_changed_in_place(planes, make):
+    from chromatix_b200.functional import propagation as P
+
+    p = make()
+    for want in (2, 3, 4):
+        out = P.transform_propagate(_field(), 100.0, 1.0, (p, p))
+        assert tuple(out.u.shape) == (16, 24)
+        # the spacing of the padded grid
+        assert planes[-1][0]["dy_out"] == pytest.approx(0.532 * 100.0 / ((16 + 2 * want) * 0.3), rel=1e-12)
+        p += 1
