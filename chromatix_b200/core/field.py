@@ -557,9 +557,9 @@ def crop(field: Field, crop_width) -> Field:
 
 def shift_grid(field: Field, shift_yx) -> Field:
     """``shift_grid`` (core/field.py:573-585): sets the origin."""
-    if type(shift_yx) is tuple and len(shift_yx) == 2 and np.shape(field.origin) in ((), (1,), (2,)):
-        return field.replace(origin=np.array(shift_yx, dtype=np.float64))
-    s = np.atleast_1d(np.asarray(shift_yx, dtype=np.float64))
+    s = np.atleast_1d(np.array(shift_yx, dtype=np.float64))
+    if s.shape == (2,) and np.shape(field.origin) in ((), (1,), (2,)):
+        return field.replace(origin=s)
     if s.size < 2:
         s = np.array([s[0], s[0]])
     if s.size != 2:
