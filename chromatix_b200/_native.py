@@ -290,20 +290,45 @@ def upload(arr: np.ndarray, device):
     return t.to(device, non_blocking=True)
 
 
+class PlanCache:
+    """Bounded map that drops its least recently used entry, safe with several
+    threads: finding an entry and marking it as used is one step, which another
+    thread's eviction cannot come between."""
+
+    def __init__(self, size: int = 64):
+        self._size, self._entries, self._lock = size, collections.OrderedDict(), threading.Lock()
+
+    def get(self, key):
+        with self._lock:
+            hit = self._entries.get(key)
+            if hit is not None:
+                self._entries.move_to_end(key)
+            return hit
+
+    def put(self, key, value):
+        with self._lock:
+            self._entries[key] = value
+            self._entries.move_to_end(key)
+            while len(self._entries) > self._size:
+                self._entries.popitem(last=False)
+
+    def clear(self):
+        with self._lock:
+            self._entries.clear()
+
+
 # (descriptor type and bytes, plane table bytes, device) -> [workspace bytes,
 # device plane table, event after its upload]: repeated calls with the same
 # geometry skip the workspace query and the host-to-device copy of their
 # plane table.  The device tables are read-only; a call waits for the upload's
 # event before its kernels read the table, until the event has been seen done.
-_TABLES = collections.OrderedDict()
-_TABLES_SIZE = 128
+_TABLES = PlanCache(128)
 
 
 def _table(key, arr, device, ws_query=None):
     torch = torch_mod()
     hit = _TABLES.get(key)
     if hit is not None:
-        _TABLES.move_to_end(key)
         ev = hit[2]
         if ev is not None and not torch.cuda.is_current_stream_capturing():
             if ev.query():
@@ -315,9 +340,8 @@ def _table(key, arr, device, ws_query=None):
     table = upload(arr, device)
     ev = torch.cuda.Event()
     ev.record(torch.cuda.current_stream(device))
-    hit = _TABLES[key] = [ws_bytes, table, ev]
-    if len(_TABLES) > _TABLES_SIZE:
-        _TABLES.popitem(last=False)
+    hit = [ws_bytes, table, ev]
+    _TABLES.put(key, hit)
     return hit
 
 

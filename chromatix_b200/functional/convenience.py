@@ -8,7 +8,6 @@ the store.
 
 from __future__ import annotations
 
-import collections
 import operator
 
 import numpy as np
@@ -160,8 +159,7 @@ def _opt_fn():
 
 
 # optical FFT call parameters -> (plan, output spacing): plans are never modified after they are built
-_OPT_PLANS = collections.OrderedDict()
-_OPT_PLANS_SIZE = 64
+_OPT_PLANS = nat.PlanCache(64)
 
 
 def _host_key(v, dtype=np.float64):
@@ -190,7 +188,6 @@ def run_optfft(field: Field, z: float, n: float, pad_width=(0, 0), crop_width=(0
            _host_key(chirp_in), _host_key(chirp_out), pupil_D, prec)
     hit = _OPT_PLANS.get(key)
     if hit is not None:
-        _OPT_PLANS.move_to_end(key)
         plan, du = hit
         return (_opt_fn().apply(field.u, plan) if nat.wants_grad(field.u) else _launch_optfft(plan, field.u)), du.copy()
     ny, nx = field.spatial_shape
@@ -232,9 +229,7 @@ def run_optfft(field: Field, z: float, n: float, pad_width=(0, 0), crop_width=(0
     out_shape = tuple(B) + (oy, ox) + ((W,) if field.chromatic else ())
     plan = _OptPlan(d, planes, tuple(field.u.shape), out_shape)
     du = np.stack([nm[2] for nm in norms])
-    _OPT_PLANS[key] = (plan, du.copy())
-    if len(_OPT_PLANS) > _OPT_PLANS_SIZE:
-        _OPT_PLANS.popitem(last=False)
+    _OPT_PLANS.put(key, (plan, du.copy()))
     if nat.wants_grad(field.u):
         u_out = _opt_fn().apply(field.u, plan)
     else:

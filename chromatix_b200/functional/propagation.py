@@ -9,7 +9,6 @@ IFFT, the crop in the last FFT's store.
 
 from __future__ import annotations
 
-import collections
 import functools
 from typing import Literal
 
@@ -137,8 +136,7 @@ class _PropPlan:
 
 # propagation call parameters -> (descriptor, plane table, output shape);
 # descriptors and tables are never modified after they are built
-_HOST_PLANS = collections.OrderedDict()
-_PLAN_CACHE_SIZE = 64
+_HOST_PLANS = nat.PlanCache(64)
 
 
 def _prop_ws(d) -> int:
@@ -360,12 +358,9 @@ def _prop2d_general(field: Field, kernel: int, zs, zshape, n, pad, kykx, shift_y
             field, zs, zshape, n, kykx, shift_yx, remove_evanescent, bandlimit, None)
         plan = _HOST_PLANS.get(key)
         if plan is None:
-            plan = _HOST_PLANS[key] = _GeneralPlan(field, kernel, zs, zshape, n, pad, kykx, shift_yx, remove_evanescent,
-                                                   bandlimit, crop_w, prec)
-            if len(_HOST_PLANS) > _PLAN_CACHE_SIZE:
-                _HOST_PLANS.popitem(last=False)
-        else:
-            _HOST_PLANS.move_to_end(key)
+            plan = _GeneralPlan(field, kernel, zs, zshape, n, pad, kykx, shift_yx, remove_evanescent, bandlimit, crop_w,
+                                prec)
+            _HOST_PLANS.put(key, plan)
         return plan.run(field)
     f = pad_field(field, (py_, px_)) if (py_ or px_) else field
     py, px = f.spatial_shape
@@ -435,7 +430,6 @@ def _run_prop2d(field: Field, kernel: int, zs, zshape, n, pad_width, kykx=(0.0, 
         field, zs, zshape, n, kykx, shift_yx, remove_evanescent, bandlimit, h_index)
     hit = _HOST_PLANS.get(key)
     if hit is not None:
-        _HOST_PLANS.move_to_end(key)
         d, planes, out_shape = hit
         return _apply_prop(_PropPlan(d, planes, tuple(field.u.shape), out_shape, field.chromatic, H), field.u)
     planes, out_batch, nb_in, nb_out = _plan_planes(field, zs, zshape, py, px, shift_yx, bandlimit, prec, h_index)
@@ -455,9 +449,7 @@ def _run_prop2d(field: Field, kernel: int, zs, zshape, n, pad_width, kykx=(0.0, 
     d.ky0, d.kx0 = float(ky0), float(kx0)
     oy, ox = (ny, nx) if mode == "same" else (py - 2 * crop[0], px - 2 * crop[1])
     out_shape = tuple(out_batch) + (oy, ox) + ((W,) if field.chromatic else ())
-    _HOST_PLANS[key] = (d, planes, out_shape)
-    if len(_HOST_PLANS) > _PLAN_CACHE_SIZE:
-        _HOST_PLANS.popitem(last=False)
+    _HOST_PLANS.put(key, (d, planes, out_shape))
     plan = _PropPlan(d, planes, tuple(field.u.shape), out_shape, field.chromatic, H)
     return _apply_prop(plan, field.u)
 
