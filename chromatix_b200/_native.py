@@ -317,30 +317,45 @@ class PlanCache:
             self._entries.clear()
 
 
-# (descriptor type and bytes, plane table bytes, device) -> [workspace bytes,
-# device plane table, event after its upload]: repeated calls with the same
-# geometry skip the workspace query and the host-to-device copy of their
-# plane table.  The device tables are read-only; a call waits for the upload's
-# event before its kernels read the table, until the event has been seen done.
+class _Table:
+    """A read-only device array kept for later calls: the stream that uploaded
+    it, the event after the upload, and the streams that may use it."""
+
+    __slots__ = ("ws_bytes", "tensor", "event", "streams")
+
+    def __init__(self, ws_bytes, tensor, event, stream):
+        self.ws_bytes, self.tensor, self.event, self.streams = ws_bytes, tensor, event, {stream}
+
+
+# (descriptor type and bytes, plane table bytes, device) -> _Table: repeated
+# calls with the same geometry skip the workspace query and the host-to-device
+# copy of their plane table.
 _TABLES = PlanCache(128)
 
 
 def _table(key, arr, device, ws_query=None):
+    """The kept device copy of ``arr`` for a call on the current stream.
+
+    The stream that uploaded it is ordered by itself.  The first call on any
+    other stream waits for the upload and names that stream to the allocator,
+    which otherwise hands an evicted table's memory to the uploading stream's
+    next allocation while a kernel still reads it.  (No event is queried: that
+    would end a capture that another thread has open.)"""
     torch = torch_mod()
     hit = _TABLES.get(key)
+    stream = stream_handle(device)
     if hit is not None:
-        ev = hit[2]
-        if ev is not None and not torch.cuda.is_current_stream_capturing():
-            if ev.query():
-                hit[2] = None
-            else:
-                torch.cuda.current_stream(device).wait_event(ev)
+        if stream not in hit.streams and not torch.cuda.is_current_stream_capturing():
+            current = torch.cuda.current_stream(device)
+            current.wait_event(hit.event)
+            hit.tensor.record_stream(current)
+            hit.streams.add(stream)
         return hit
     ws_bytes = int(ws_query()) if ws_query is not None else 0
-    table = upload(arr, device)
+    tensor = upload(arr, device)
     ev = torch.cuda.Event()
     ev.record(torch.cuda.current_stream(device))
-    hit = [ws_bytes, table, ev]
+    hit = _Table(ws_bytes, tensor, ev, stream)
     _TABLES.put(key, hit)
     return hit
 
@@ -350,13 +365,13 @@ def device_table(desc, planes: np.ndarray, device, ws_query):
     the ctypes struct ``desc``; ``ws_query(desc)`` returns the workspace size."""
     key = (type(desc).__name__, bytes(desc), planes.tobytes(), device_index(device))
     hit = _table(key, np.ascontiguousarray(planes).view(np.uint8).reshape(-1), device, lambda: ws_query(desc))
-    return hit[0], hit[1]
+    return hit.ws_bytes, hit.tensor
 
 
 def constant(arr: np.ndarray, device):
     """Device copy of a small read-only host array (per-wavelength factors, densities), kept by its content."""
     key = ("constant", arr.dtype.str, arr.shape, arr.tobytes(), device_index(device))
-    return _table(key, arr, device)[1]
+    return _table(key, arr, device).tensor
 
 
 def to_device_bytes(arr: np.ndarray, device):
