@@ -281,13 +281,15 @@ def workspace(nbytes: int, device):
     return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
 
 
+def _pinned(arr: np.ndarray):
+    return torch_mod().from_numpy(np.ascontiguousarray(arr)).pin_memory()
+
+
 def upload(arr: np.ndarray, device):
     """Host array -> device tensor through page-locked memory, asynchronous on
     the current stream: the host does not wait for the stream (a pageable
     blocking copy would synchronise it, serialising host and device)."""
-    torch = torch_mod()
-    t = torch.from_numpy(np.ascontiguousarray(arr)).pin_memory()
-    return t.to(device, non_blocking=True)
+    return _pinned(arr).to(device, non_blocking=True)
 
 
 class PlanCache:
@@ -344,8 +346,10 @@ def _table(key, arr, device, ws_query=None):
     torch = torch_mod()
     hit = _TABLES.get(key)
     stream = stream_handle(device)
+    if torch.cuda.is_current_stream_capturing():
+        return _captured_table(key, hit, arr, device, ws_query)
     if hit is not None:
-        if stream not in hit.streams and not torch.cuda.is_current_stream_capturing():
+        if stream not in hit.streams:
             current = torch.cuda.current_stream(device)
             current.wait_event(hit.event)
             hit.tensor.record_stream(current)
@@ -358,6 +362,26 @@ def _table(key, arr, device, ws_query=None):
     hit = _Table(ws_bytes, tensor, ev, stream)
     _TABLES.put(key, hit)
     return hit
+
+
+# What captured graphs read whenever they are replayed, by the same keys: the
+# kept tables, and the page-locked sources of uploads that were captured.  A
+# graph holds raw pointers and does not say when it is gone, so these are not
+# dropped: some hundred bytes for each geometry that was ever captured.
+_CAPTURED = {}
+
+
+def _captured_table(key, hit, arr, device, ws_query):
+    """:func:`_table` inside a capture.  A table uploaded before it is not freed
+    from now on.  An upload made here runs with each replay of the graph, not
+    now: it serves this call alone."""
+    hit = _CAPTURED.get((key, "table"), hit)
+    if hit is not None:
+        return _CAPTURED.setdefault((key, "table"), hit)
+    source = _CAPTURED.get((key, "source"))
+    if source is None:
+        source = _CAPTURED.setdefault((key, "source"), _pinned(arr))
+    return _Table(int(ws_query()) if ws_query is not None else 0, source.to(device, non_blocking=True), None, None)
 
 
 def device_table(desc, planes: np.ndarray, device, ws_query):

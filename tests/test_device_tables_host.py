@@ -64,6 +64,8 @@ def gpu(monkeypatch):
     monkeypatch.setattr(nat, "device_index", lambda device=None: 0)
     monkeypatch.setattr(nat, "stream_handle", lambda device=None: fake.handle)
     monkeypatch.setattr(nat, "upload", lambda arr, device: Table(arr))
+    if hasattr(nat, "_CAPTURED"):
+        monkeypatch.setattr(nat, "_CAPTURED", {})
     for name in ("_TABLES", "_CONSTANTS"):
         if hasattr(nat, name):
             monkeypatch.setattr(nat, name, nat.PlanCache(128))
@@ -98,3 +100,66 @@ def test_use_on_another_stream(gpu, make):
     gpu.is_in(1)
     assert make(1.0) is t
     assert t.recorded == [2, 3] and gpu.log == [("wait", 2, 1), ("wait", 3, 1)]
+
+
+@pytest.mark.parametrize("make", [constant, plane_table])
+def test_first_call_inside_a_capture(gpu, monkeypatch, make):
+    """A table uploaded inside a capture holds its values only once the graph
+    has run: later calls get their own, and what the graph copies from lives on."""
+    hosts = []
+
+    class Host:
+        def __init__(self, arr):
+            self.arr = np.array(arr)
+            hosts.append(weakref.ref(self))
+
+        def to(self, device, non_blocking=False):
+            return Table(self.arr)
+
+    monkeypatch.setattr(nat, "_pinned", Host, raising=False)
+    gpu.is_in(5, capturing=True)
+    t = make(3.0)
+    gpu.is_in(5)
+    eager = make(3.0)
+    assert eager is not t and make(3.0) is eager
+    del t
+    gc.collect()
+    assert len(hosts) == 1 and hosts[0]() is not None
+    # a second graph copies from the same place
+    nat._TABLES.clear(), nat._CONSTANTS.clear() if hasattr(nat, "_CONSTANTS") else None
+    gpu.is_in(5, capturing=True)
+    make(3.0)
+    assert len(hosts) == 1
+
+
+@pytest.mark.parametrize("make", [constant, plane_table])
+def test_table_of_a_captured_graph_outlives_eviction(gpu, make):
+    t = make(-1.0)
+    addr = weakref.ref(t)
+    gpu.is_in(5, capturing=True)
+    assert make(-1.0) is t
+    assert t.recorded == [] and gpu.log == []
+    gpu.is_in(1)
+    del t
+    for k in range(400):
+        make(float(k))
+    gc.collect()
+    assert addr() is not None
+    # a later graph of the same geometry does not displace it
+    make(-1.0)
+    gpu.is_in(5, capturing=True)
+    make(-1.0)
+    gpu.is_in(1)
+    for k in range(400):
+        make(float(k))
+    gc.collect()
+    assert addr() is not None
+
+
+@pytest.mark.parametrize("make", [constant, plane_table])
+def test_eviction_frees_a_table(gpu, make):
+    addr = weakref.ref(make(-1.0))
+    for k in range(400):
+        make(float(k))
+    gc.collect()
+    assert addr() is None
