@@ -333,9 +333,12 @@ class _Table:
 # calls with the same geometry skip the workspace query and the host-to-device
 # copy of their plane table.
 _TABLES = PlanCache(128)
+# (content, device) -> _Table: a cache of their own, so that changing densities
+# or phase factors do not displace the plane tables.
+_CONSTANTS = PlanCache(128)
 
 
-def _table(key, arr, device, ws_query=None):
+def _table(cache, key, arr, device, ws_query=None):
     """The kept device copy of ``arr`` for a call on the current stream.
 
     The stream that uploaded it is ordered by itself.  The first call on any
@@ -344,7 +347,7 @@ def _table(key, arr, device, ws_query=None):
     next allocation while a kernel still reads it.  (No event is queried: that
     would end a capture that another thread has open.)"""
     torch = torch_mod()
-    hit = _TABLES.get(key)
+    hit = cache.get(key)
     stream = stream_handle(device)
     if torch.cuda.is_current_stream_capturing():
         return _captured_table(key, hit, arr, device, ws_query)
@@ -360,7 +363,7 @@ def _table(key, arr, device, ws_query=None):
     ev = torch.cuda.Event()
     ev.record(torch.cuda.current_stream(device))
     hit = _Table(ws_bytes, tensor, ev, stream)
-    _TABLES.put(key, hit)
+    cache.put(key, hit)
     return hit
 
 
@@ -388,14 +391,14 @@ def device_table(desc, planes: np.ndarray, device, ws_query):
     """(workspace bytes, device copy of ``planes``) for a launch described by
     the ctypes struct ``desc``; ``ws_query(desc)`` returns the workspace size."""
     key = (type(desc).__name__, bytes(desc), planes.tobytes(), device_index(device))
-    hit = _table(key, np.ascontiguousarray(planes).view(np.uint8).reshape(-1), device, lambda: ws_query(desc))
+    hit = _table(_TABLES, key, np.ascontiguousarray(planes).view(np.uint8).reshape(-1), device, lambda: ws_query(desc))
     return hit.ws_bytes, hit.tensor
 
 
 def constant(arr: np.ndarray, device):
     """Device copy of a small read-only host array (per-wavelength factors, densities), kept by its content."""
     key = ("constant", arr.dtype.str, arr.shape, arr.tobytes(), device_index(device))
-    return _table(key, arr, device).tensor
+    return _table(_CONSTANTS, key, arr, device).tensor
 
 
 def to_device_bytes(arr: np.ndarray, device):

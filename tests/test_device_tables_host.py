@@ -64,11 +64,9 @@ def gpu(monkeypatch):
     monkeypatch.setattr(nat, "device_index", lambda device=None: 0)
     monkeypatch.setattr(nat, "stream_handle", lambda device=None: fake.handle)
     monkeypatch.setattr(nat, "upload", lambda arr, device: Table(arr))
-    if hasattr(nat, "_CAPTURED"):
-        monkeypatch.setattr(nat, "_CAPTURED", {})
+    monkeypatch.setattr(nat, "_CAPTURED", {})
     for name in ("_TABLES", "_CONSTANTS"):
-        if hasattr(nat, name):
-            monkeypatch.setattr(nat, name, nat.PlanCache(128))
+        monkeypatch.setattr(nat, name, nat.PlanCache(128))
     return fake
 
 
@@ -126,7 +124,8 @@ def test_first_call_inside_a_capture(gpu, monkeypatch, make):
     gc.collect()
     assert len(hosts) == 1 and hosts[0]() is not None
     # a second graph copies from the same place
-    nat._TABLES.clear(), nat._CONSTANTS.clear() if hasattr(nat, "_CONSTANTS") else None
+    nat._TABLES.clear()
+    nat._CONSTANTS.clear()
     gpu.is_in(5, capturing=True)
     make(3.0)
     assert len(hosts) == 1
@@ -163,3 +162,11 @@ def test_eviction_frees_a_table(gpu, make):
         make(float(k))
     gc.collect()
     assert addr() is None
+
+
+def test_constants_do_not_displace_plane_tables(gpu):
+    """Many densities or phase factors leave the plane tables where they are."""
+    t = plane_table(1.0)
+    for k in range(400):
+        constant(float(k))
+    assert plane_table(1.0) is t
