@@ -300,10 +300,10 @@ extern "C" cx_status cx_multislice_forward(const cx_ms_desc* d, const void* u_in
   return ms_rows(a, st);
 }
 
-extern "C" cx_status cx_multislice_backward(const cx_ms_desc* d, const float* dn, const float* ab,
-                                            const void* checkpoints, const void* grad_out, float* grad_dn,
-                                            float* grad_ab, void* grad_u_in, void* workspace, size_t workspace_bytes,
-                                            cx_stream_t stream) {
+// overlap: the recomputation on the second stream, where there is one
+static cx_status ms_backward(const cx_ms_desc* d, const float* dn, const float* ab, const void* checkpoints,
+                             const void* grad_out, float* grad_dn, float* grad_ab, void* grad_u_in, void* workspace,
+                             size_t workspace_bytes, cx_stream_t stream, bool overlap) {
   MsPlan p;
   cx_status s = ms_plan(d, &p);
   if (s != CX_OK) return s;
@@ -396,6 +396,7 @@ extern "C" cx_status cx_multislice_backward(const cx_ms_desc* d, const float* dn
     for (int i = i1 - 1; i >= i0; --i) {
       g.slice = i;
       g.rec_u = recs + (size_t)(i - i0) * stride;
+      g.rec_new = !last && i == i1 - 1;
       g.gdn = grad_dn + (size_t)i * d->ny * d->nx;
       g.gab = grad_ab + (size_t)i * d->ny * d->nx;
       if ((e = ms_rows(g, q)) != CX_OK) return e;
@@ -404,7 +405,7 @@ extern "C" cx_status cx_multislice_backward(const cx_ms_desc* d, const float* dn
     return CX_OK;
   };
 
-  cudaStream_t rs = ms_side_stream();
+  cudaStream_t rs = overlap ? ms_side_stream() : nullptr;
   cudaEvent_t ev[4] = {};  // fork, recomputed (two halves), adjoint done
   int made = 0;
   if (rs && rs != st) {
@@ -456,4 +457,20 @@ extern "C" cx_status cx_multislice_backward(const cx_ms_desc* d, const float* dn
     return ms_rows(g, st);
   }
   return CX_OK;
+}
+
+extern "C" cx_status cx_multislice_backward(const cx_ms_desc* d, const float* dn, const float* ab,
+                                            const void* checkpoints, const void* grad_out, float* grad_dn,
+                                            float* grad_ab, void* grad_u_in, void* workspace, size_t workspace_bytes,
+                                            cx_stream_t stream) {
+  return ms_backward(d, dn, ab, checkpoints, grad_out, grad_dn, grad_ab, grad_u_in, workspace, workspace_bytes, stream,
+                     true);
+}
+
+extern "C" cx_status cx_multislice_backward_one_stream(const cx_ms_desc* d, const float* dn, const float* ab,
+                                                       const void* checkpoints, const void* grad_out, float* grad_dn,
+                                                       float* grad_ab, void* grad_u_in, void* workspace,
+                                                       size_t workspace_bytes, cx_stream_t stream) {
+  return ms_backward(d, dn, ab, checkpoints, grad_out, grad_dn, grad_ab, grad_u_in, workspace, workspace_bytes, stream,
+                     false);
 }

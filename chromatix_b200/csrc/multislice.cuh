@@ -31,6 +31,7 @@ struct MsArgs {
   double lam, dz;
   float kdz_f;          // 2 pi dz / lam rounded once to float
   float kdz_lo;         // and what the rounding left
+  int rec_new;          // MS_BWD: rec_u comes from a recomputation that this launch follows
   int sy, sx, oy, ox;   // MS_LOAD source: (sy, sx) matrix placed at offset (oy, ox) of the padded grid
   const float* dn;      // (D, ny, nx) refractive-index change (unpadded)
   const float* ab;      // (D, ny, nx) absorption (unpadded)

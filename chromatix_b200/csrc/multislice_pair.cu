@@ -11,8 +11,9 @@ static cx_status launch_ms_rows_pair_mode(const MsArgs& a, cudaStream_t st) {
   CX_CUDA_TRY(f.err);
   const int rows = MODE == MS_FINAL ? a.ny : a.py;
   // MS_LOAD follows the kernel that fills the propagator, which the next pass reads before it waits, and MS_FLUOR
-  // the one that draws the phases: those two wait for their predecessor as a whole
-  const bool pdl = MODE != MS_LOAD && MODE != MS_FLUOR;
+  // the one that draws the phases: those two wait for their predecessor as a whole.  So does the first MS_BWD after
+  // a recomputation: it copies a record before pdl_wait, and the pass that wrote it may be its predecessor.
+  const bool pdl = MODE != MS_LOAD && MODE != MS_FLUOR && !(MODE == MS_BWD && a.rec_new);
   CX_CUDA_TRY(launch_kernel(k, (rows + 1) / 2, C::THREADS, C::SMEM, st, pdl, a));
   return CX_OK;
 }

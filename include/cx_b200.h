@@ -266,7 +266,7 @@ typedef struct {
   int32_t n_slices;          /* D */
   int32_t precision;         /* cx_precision */
   int32_t remove_evanescent, bandlimit;  /* slice propagator options */
-  int32_t checkpoint_every;  /* K; <= 0: D where D + 1 padded planes take at most 4 GiB, else ceil(sqrt(D)) */
+  int32_t checkpoint_every;  /* K; <= 0: D where D + 1 padded planes of this call take at most 4 GiB, else ceil(sqrt(D)) */
   double n_medium, wavelength, dy, dx;
   double dz;                 /* thickness_per_slice */
   double reverse_distance;   /* defocus back by this distance */
@@ -287,6 +287,12 @@ cx_status cx_multislice_forward(const cx_ms_desc* d, const void* u_in, const flo
 cx_status cx_multislice_backward(const cx_ms_desc* d, const float* dn, const float* abs_, const void* checkpoints,
                                  const void* grad_out, float* grad_dn, float* grad_abs, void* grad_u_in,
                                  void* workspace, size_t workspace_bytes, cx_stream_t stream);
+/* The same on `stream` alone, the recomputation before each segment's adjoint: what cx_multislice_backward
+ * does where its second stream cannot be created.  The same gradients, bit for bit. */
+cx_status cx_multislice_backward_one_stream(const cx_ms_desc* d, const float* dn, const float* abs_,
+                                            const void* checkpoints, const void* grad_out, float* grad_dn,
+                                            float* grad_abs, void* grad_u_in, void* workspace, size_t workspace_bytes,
+                                            cx_stream_t stream);
 
 /* ---------------------------------------------------------------------------
  * Chirp-Z transform along one axis (Bluestein)
