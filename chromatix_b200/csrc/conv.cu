@@ -74,8 +74,12 @@ static cx_status conv_plan(const cx_conv_desc* d, ConvArgs* a, int* zc, size_t* 
   *zc = c;
   *t_bytes = ((plane_t * c) + 255) & ~(size_t)255;
   const size_t st_bytes = ((sizeof(float2) * (size_t)a->NC * a->P) + 255) & ~(size_t)255;
+  // CTAs that can share a column of the pair pass: G / NC rounded up, and one
+  const int ctas = d->reduce && conv_on_pairs(a->M, a->P) ? conv_pair_col_ctas(a->P) : 0;
+  const int share = (ctas + a->NC - 1) / a->NC + 1;
+  a->slabs = ctas <= a->NC || c <= 2 ? 1 : (share < c ? share : c);
   const size_t u_bytes = ((sizeof(float2) * (size_t)a->NC * d->h) + 255) & ~(size_t)255;
-  *total = *t_bytes + st_bytes + u_bytes;
+  *total = *t_bytes + st_bytes + u_bytes + (a->slabs > 1 ? a->slabs * st_bytes : 0);
   return CX_OK;
 }
 
@@ -115,6 +119,7 @@ extern "C" cx_status cx_conv2d_same(const cx_conv_desc* d, const float* sample, 
   a.T = reinterpret_cast<float2*>(ws);
   a.St = reinterpret_cast<float2*>(ws + tb);
   a.U = reinterpret_cast<float2*>(ws + tb + (((sizeof(float2) * (size_t)a.NC * a.P) + 255) & ~(size_t)255));
+  a.part = a.slabs > 1 ? a.U + (((sizeof(float2) * (size_t)a.NC * d->h) + 255) & ~(size_t)255) / sizeof(float2) : nullptr;
   a.a = sample;
   a.b = kernel;
   const size_t st_bytes = sizeof(float2) * (size_t)a.NC * a.P;
@@ -124,9 +129,10 @@ extern "C" cx_status cx_conv2d_same(const cx_conv_desc* d, const float* sample, 
   const int groups = d->reduce ? 1 : d->n_planes;
   for (int g = 0; g < groups; ++g) {
     const int p_lo = d->reduce ? 0 : g, p_hi = d->reduce ? d->n_planes : g + 1;
-    CX_CUDA_TRY(cudaMemsetAsync(a.St, 0, st_bytes, st));
+    if (a.slabs == 1) CX_CUDA_TRY(cudaMemsetAsync(a.St, 0, st_bytes, st));
     for (int z0 = p_lo; z0 < p_hi; z0 += zc) {
       a.z0 = z0;
+      a.fresh = z0 == p_lo;
       a.zc = (p_hi - z0) < zc ? (p_hi - z0) : zc;
       if (pairs) {
         if ((s = conv_dispatch_rows_pair(a.M, a, st)) != CX_OK) return s;

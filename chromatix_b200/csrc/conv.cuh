@@ -45,6 +45,9 @@ struct ConvArgs {
   int kh, kw;             // kernel (PSF) plane shape
   int HB;                 // rows per tile block of T: max(h, kh)
   int ldY;                // pair passes (conv_pair.cuh): rows of T's columns, HB rounded up to even
+  int slabs;              // CTAs that can share a column of the pair column pass; 1: at most two
+  int fresh;              // (slabs > 1) the first chunk: St holds nothing yet
+  float2* part;           // their partial sums (slabs, NC, P), where slabs > 1
   int NT, vt_shift;       // column tiles of T and their width VT = 1 << vt_shift (>= 4, a multiple of the column pass's V)
   int P, Q, M, NC;        // transform lengths, M = Q / 2, NC = M + 1
   int z0, zc;             // plane chunk
@@ -345,6 +348,7 @@ __global__ void __launch_bounds__(ConvFinCfg<M>::THREADS, ConvFinCfg<M>::MINB) k
 // the passes on (sample, kernel) pairs (conv_pair.cuh)
 cx_status conv_dispatch_rows_pair(int m, const ConvArgs& a, cudaStream_t st);
 cx_status conv_dispatch_cols_pair(int p, const ConvArgs& a, cudaStream_t st);
+int conv_pair_col_ctas(int p);  // the largest grid of the column pass for length p
 cx_status conv_dispatch_rows(int m, const ConvArgs& a, cudaStream_t st);
 int conv_col_tile(int p);  // the column pass's tile width V for length p (0: unsupported)
 cx_status conv_dispatch_cols(int p, const ConvArgs& a, cudaStream_t st);

@@ -13,13 +13,31 @@ static cx_status launch_conv_rows_pair(const ConvArgs& a, cudaStream_t st) {
   return CX_OK;
 }
 
-template <int P>
+template <int P, bool SLAB>
 static cx_status launch_conv_cols_pair(const ConvArgs& a, cudaStream_t st) {
   using C = ConvPairCols<P>;
-  auto k = k_conv_cols_pair<P>;
-  k<<<persistent_grid(k, C::THREADS, C::SMEM, (long)a.NC * a.zc), C::THREADS, C::SMEM, st>>>(a);
+  auto k = k_conv_cols_pair<P, SLAB>;
+  const long units = (long)a.NC * a.zc;
+  const int grid = persistent_grid(k, C::THREADS, C::SMEM, units < C::CTAS ? units : C::CTAS);
+  k<<<grid, C::THREADS, C::SMEM, st>>>(a);
   CX_LAUNCH_CHECK();
+  if constexpr (SLAB) {
+    const long blocks = ((long)a.NC * P + 255) / 256, most = (long)sm_count() * 8;
+    k_conv_sum<<<(int)(blocks < most ? blocks : most), 256, 0, st>>>(a, grid);
+    CX_LAUNCH_CHECK();
+  }
   return CX_OK;
+}
+
+int conv_pair_col_ctas(int p) {
+  switch (p) {
+#define CX_CASE_(N, ...) \
+  case N:                \
+    return ConvPairCols<N>::CTAS;
+    CX_PAIR_PLANS_4096(CX_CASE_)
+#undef CX_CASE_
+  }
+  return 0;
 }
 
 cx_status conv_dispatch_rows_pair(int m, const ConvArgs& a, cudaStream_t st) {
@@ -38,7 +56,7 @@ cx_status conv_dispatch_cols_pair(int p, const ConvArgs& a, cudaStream_t st) {
   switch (p) {
 #define CX_CASE_(N, ...) \
   case N:                \
-    return launch_conv_cols_pair<N>(a, st);
+    return a.slabs > 1 ? launch_conv_cols_pair<N, true>(a, st) : launch_conv_cols_pair<N, false>(a, st);
     CX_PAIR_PLANS_4096(CX_CASE_)
 #undef CX_CASE_
   }

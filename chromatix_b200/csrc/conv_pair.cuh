@@ -114,6 +114,11 @@ __global__ void __launch_bounds__(ConvPairRows<M>::THREADS, ConvPairRows<M>::MIN
 // --------------------------------------------------------------------------
 // Work units (column, plane) split in equal contiguous ranges over the
 // resident CTAs (no last wave); a range's sums go to St when it leaves a column.
+// With at least as many columns as CTAs a column belongs to two CTAs at most,
+// and 0 + a + b is the same in both orders.  With fewer (images of up to about
+// a thousand pixels) more CTAs share one, and the order in which they finish
+// would decide the rounding: each then stores its sum to a slab of its own,
+// and k_conv_sum adds a column's slabs to St in order.
 // The first stage's twiddles stay in registers: 6 KB less shared memory let a
 // third CTA per SM in at 3072 (64 planes: 1347 -> 1284 us; 4096: 2404 -> 2271;
 // 512 to 2560: within 3 %).
@@ -129,10 +134,15 @@ struct ConvPairCols {
   // up to 20 warps per SM, as far as their shared memory goes
   static constexpr int FIT = (int)(227 * 1024 / (SMEM + 1024));
   static constexpr int MINB = 20 / WARPS < 1 || FIT < 1 ? 1 : (20 / WARPS < FIT ? 20 / WARPS : FIT);
+  static constexpr int CTAS = 148 * MINB;
   static_assert(SMEM <= 227 * 1024, "convolution column does not fit one CTA");
 };
 
-template <int P>
+// the range that holds unit u of `units` in `ctas` ranges
+__device__ __forceinline__ long conv_owner(long u, long units, long ctas) { return ((u + 1) * ctas - 1) / units; }
+
+// SLAB: a.slabs > 1 (in a kernel of its own: the other one has no registers to spare, 1907 -> 1951 us at 128 x 1024^2)
+template <int P, bool SLAB>
 __global__ void __launch_bounds__(ConvPairCols<P>::THREADS, ConvPairCols<P>::MINB) k_conv_cols_pair(ConvArgs a) {
   using C = ConvPairCols<P>;
   using F = typename C::F;
@@ -157,15 +167,19 @@ __global__ void __launch_bounds__(ConvPairCols<P>::THREADS, ConvPairCols<P>::MIN
       return {make_float2(v.x, v.y), make_float2(v.z, v.w)};
     };
     const bool leave = u + 1 == u1 || zl + 1 == a.zc;
-    float2* col = a.St + (size_t)kc * a.P;
+    float2* col = (SLAB ? a.part : a.St) + (size_t)kc * a.P;
+    // this CTA's number among those of the column
+    if (SLAB && leave) col += (blockIdx.x - conv_owner((long)kc * a.zc, units, gridDim.x)) * a.NC * a.P;
     // acc[k] belongs to one lane: no barrier between its updates
     auto out = [&](int k, c2 v) {
       float2 p = cmul(make_float2(v.re.x, v.im.x), make_float2(v.re.y, v.im.y));
       if (!fresh) p = cadd(acc[k], p);
-      if (leave)
-        atomicAdd(col + k, p);
-      else
+      if (!leave)
         acc[k] = p;
+      else if (SLAB)
+        col[k] = p;
+      else
+        atomicAdd(col + k, p);
     };
     __syncthreads();  // the previous column has been read
     // rows >= HB are zero and P >= 2 HB
@@ -173,6 +187,21 @@ __global__ void __launch_bounds__(ConvPairCols<P>::THREADS, ConvPairCols<P>::MIN
     F::template inner<false>(s, tw, t, sync);
     F::template last<false>(s, t, out);
     fresh = leave;
+  }
+}
+
+// St[kc][k] (+)= the slabs of column kc, one thread per element (the whole sum
+// of 64 planes of 256^2 with its 6 MB of slabs: 84 -> 88 us, of 48 x 768^2 454 ->
+// 461; with the slabs added in the final pass's loader 110 and 492).
+static __global__ void k_conv_sum(ConvArgs a, int ctas) {
+  const long units = (long)a.NC * a.zc, n = (long)a.NC * a.P;
+  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
+    const long u = e / a.P * a.zc;
+    const int count = (int)(conv_owner(u + a.zc - 1, units, ctas) - conv_owner(u, units, ctas)) + 1;
+    float2 v = a.fresh ? make_float2(0.f, 0.f) : a.St[e];
+#pragma unroll 8
+    for (int s = 0; s < count; ++s) v = cadd(v, a.part[s * n + e]);
+    a.St[e] = v;
   }
 }
 
