@@ -186,10 +186,12 @@ static void psf_cols_box(const cx_psf_desc* d, const cx_psf_spectrum* spec, int 
 // pass on three planes of a 3 x 1280^2 stack, and the launches' ramps and last
 // waves cost more than the spectra's way through HBM (64 planes, chunk in MiB:
 // 44 2023 us, 64 2103, 132 1930, 264 1753, 600 1702, all planes at once 1670).
+// CX_PSF_L2_MB, the name from when the chunk was sized to the L2, still counts.
 static size_t psf_chunk_budget() {
   static size_t cached = 0;
   if (!cached) {
     const char* e = getenv("CX_PSF_CHUNK_MB");
+    if (!e) e = getenv("CX_PSF_L2_MB");
     const long mb = e ? atol(e) : 512;
     cached = (size_t)(mb > 0 ? mb : 512) << 20;
   }
