@@ -12,7 +12,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 QUERY = """
 from chromatix_b200 import _native as nat
 d = nat.cx_psf_desc()
-d.ny, d.nx, d.n_wv, d.n_z = 1280, 1280, 3, 64
+d.ny, d.nx, d.n_wv, d.n_z, d.f_lens = 1280, 1280, 3, 64, 1.0
 b = nat.c_size_t(0)
 nat.check(nat.lib().cx_psf_workspace_size(d, b))
 print(b.value)
