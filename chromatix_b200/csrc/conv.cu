@@ -113,7 +113,7 @@ extern "C" cx_status cx_conv2d_same(const cx_conv_desc* d, const float* sample, 
     set_error("workspace too small: %zu < %zu", workspace_bytes, total);
     return CX_ERR_WORKSPACE;
   }
-  if ((s = ensure_twiddles(&a.twg)) != CX_OK) return s;
+  if ((s = ensure_twiddles(&a.twg, true)) != CX_OK) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(workspace);
   a.T = reinterpret_cast<float2*>(ws);

@@ -111,7 +111,7 @@ extern "C" cx_status cx_czt(const cx_czt_desc* d, const void* x, void* y, void* 
     return CX_ERR_WORKSPACE;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if ((s = ensure_twiddles(&a.twg)) != CX_OK) return s;
+  if ((s = ensure_twiddles(&a.twg, true)) != CX_OK) return s;
   float2* c = static_cast<float2*>(workspace);
   float2* chat = c + a.L;
   k_czt_filter<<<(a.L + 255) / 256, 256, 0, st>>>(c, a.n, a.m, a.L, a.tw, a.lw);
@@ -178,7 +178,7 @@ extern "C" cx_status cx_czt_noalloc(const cx_czt_desc* d, const void* x, void* y
     return CX_ERR_INVALID;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if ((s = ensure_twiddles(&a.twg)) != CX_OK) return s;
+  if ((s = ensure_twiddles(&a.twg, true)) != CX_OK) return s;
   float2* c = nullptr;
   if ((s = czt_noalloc_scratch(&c)) != CX_OK) return s;
   float2* chat = c + a.L;

@@ -219,7 +219,7 @@ extern "C" cx_status cx_czt_propagate(const cx_czt_prop_desc* d, const void* u_i
   CztArgs yu[2];
   if (d->method == 1) {
     const float2* twg = nullptr;
-    if ((s = ensure_twiddles(&twg)) != CX_OK) return s;
+    if ((s = ensure_twiddles(&twg, true)) != CX_OK) return s;
     const int Ls[2] = {L.Ly, L.Lx};
     for (int k = 0; k < 2; ++k) {
       const int n = P[k];

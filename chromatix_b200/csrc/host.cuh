@@ -95,7 +95,9 @@ constexpr int kTwTotal = tw_total();
 // Device twiddle tables (twiddles.cu): ensure_twiddles() uploads them (host
 // FP64 values rounded to float) once per device, synchronously, and returns
 // their device address; kernels receive it in their argument structs.
-cx_status ensure_twiddles(const float2** table);
+// unit: the tables rounded to unit modulus on average (see twiddles.cu), for
+// the propagations, optical FFTs, chirp-Z transforms and convolutions.
+cx_status ensure_twiddles(const float2** table, bool unit = false);
 
 // The real-expanded forward DFT matrices of the split-precision tensor-core
 // transforms (lengths 32 and 40): 2R x 2R, K-major canonical layout, FP16 hi

@@ -64,7 +64,7 @@ extern "C" cx_status cx_optical_fft(const cx_optfft_desc* d, const cx_fft_plane*
   }
   a.planes = planes_dev;
   a.H = nullptr;
-  if ((s = ensure_twiddles(&a.twg)) != CX_OK) return s;
+  if ((s = ensure_twiddles(&a.twg, d->precision == CX_PREC_ACCURATE)) != CX_OK) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   float2* T = static_cast<float2*>(workspace);
   if ((s = opt_dispatch_rows(a.px, static_cast<const float2*>(u_in), T, a, st)) != CX_OK) return s;
@@ -88,7 +88,7 @@ extern "C" cx_status cx_optical_fft_h(const cx_optfft_desc* d, const cx_fft_plan
   }
   a.planes = planes_dev;
   a.H = static_cast<const float2*>(H);
-  if ((s = ensure_twiddles(&a.twg)) != CX_OK) return s;
+  if ((s = ensure_twiddles(&a.twg, d->precision == CX_PREC_ACCURATE)) != CX_OK) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   float2* T = static_cast<float2*>(workspace);
   if ((s = opt_dispatch_rows(a.px, static_cast<const float2*>(u_in), T, a, st)) != CX_OK) return s;

@@ -138,7 +138,7 @@ extern "C" cx_status cx_prop2d(const cx_prop2d_desc* d, const cx_plane* planes_d
   }
   a.planes = planes_dev;
   a.H = static_cast<const float2*>(H);
-  if ((s = ensure_twiddles(&a.twg)) != CX_OK) return s;
+  if ((s = ensure_twiddles(&a.twg, d->precision == CX_PREC_ACCURATE)) != CX_OK) return s;
   float2* T = static_cast<float2*>(workspace);
   float2* T2 = reinterpret_cast<float2*>(static_cast<char*>(workspace) + align256(ws_T_bytes(a)));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -170,7 +170,7 @@ extern "C" cx_status cx_prop2d_ptrs(const cx_prop2d_desc* d, const cx_plane* pla
   a.H = static_cast<const float2*>(H);
   a.in_ptrs = reinterpret_cast<const float2* const*>(u_in_ptrs_dev);
   a.out_ptrs = reinterpret_cast<float2* const*>(u_out_ptrs_dev);
-  if ((s = ensure_twiddles(&a.twg)) != CX_OK) return s;
+  if ((s = ensure_twiddles(&a.twg, d->precision == CX_PREC_ACCURATE)) != CX_OK) return s;
   float2* T = static_cast<float2*>(workspace);
   float2* T2 = reinterpret_cast<float2*>(static_cast<char*>(workspace) + align256(ws_T_bytes(a)));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
