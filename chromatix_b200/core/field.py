@@ -557,9 +557,10 @@ def crop(field: Field, crop_width) -> Field:
 
 def shift_grid(field: Field, shift_yx) -> Field:
     """``shift_grid`` (core/field.py:573-585): sets the origin."""
-    s = np.atleast_1d(np.array(shift_yx, dtype=np.float64))
+    s = np.array(shift_yx, dtype=np.float64)
     if s.shape == (2,) and np.shape(field.origin) in ((), (1,), (2,)):
         return field.replace(origin=s)
+    s = np.atleast_1d(s)
     if s.size < 2:
         s = np.array([s[0], s[0]])
     if s.size != 2:
