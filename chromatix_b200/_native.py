@@ -344,6 +344,11 @@ _TABLES = PlanCache(128)
 _CONSTANTS = PlanCache(128)
 
 
+def _as_bytes(arr):
+    """Structured arrays as raw bytes, which torch takes; others as they are."""
+    return np.ascontiguousarray(arr).view(np.uint8).reshape(-1) if arr.dtype.names else arr
+
+
 def _table(cache, key, arr, device, ws_query=None):
     """The kept device copy of ``arr`` for a call on the current stream.
 
@@ -354,9 +359,9 @@ def _table(cache, key, arr, device, ws_query=None):
     would end a capture that another thread has open.)"""
     torch = torch_mod()
     hit = cache.get(key)
-    if torch.cuda.is_current_stream_capturing():
-        return _captured_table(key, hit, arr, device, ws_query)
     stream = stream_handle(device)
+    if stream != 0 and torch.cuda.is_current_stream_capturing():  # (the default stream cannot be captured)
+        return _captured_table(key, hit, arr, device, ws_query)
     if hit is not None:
         if stream not in hit.streams:
             current = torch.cuda.current_stream(device)
@@ -365,7 +370,7 @@ def _table(cache, key, arr, device, ws_query=None):
             hit.streams.add(stream)
         return hit
     ws_bytes = int(ws_query()) if ws_query is not None else 0
-    tensor = upload(arr, device)
+    tensor = upload(_as_bytes(arr), device)
     ev = torch.cuda.Event()
     ev.record(torch.cuda.current_stream(device))
     hit = _Table(ws_bytes, tensor, ev, stream)
@@ -389,7 +394,7 @@ def _captured_table(key, hit, arr, device, ws_query):
         return _CAPTURED.setdefault((key, "table"), hit)
     source = _CAPTURED.get((key, "source"))
     if source is None:
-        source = _CAPTURED.setdefault((key, "source"), _pinned(arr))
+        source = _CAPTURED.setdefault((key, "source"), _pinned(_as_bytes(arr)))
     return _Table(int(ws_query()) if ws_query is not None else 0, source.to(device, non_blocking=True), None, None)
 
 
@@ -397,7 +402,7 @@ def device_table(desc, planes: np.ndarray, device, ws_query):
     """(workspace bytes, device copy of ``planes``) for a launch described by
     the ctypes struct ``desc``; ``ws_query(desc)`` returns the workspace size."""
     key = (type(desc).__name__, bytes(desc), planes.tobytes(), device_index(device))
-    hit = _table(_TABLES, key, np.ascontiguousarray(planes).view(np.uint8).reshape(-1), device, lambda: ws_query(desc))
+    hit = _table(_TABLES, key, planes, device, lambda: ws_query(desc))
     return hit.ws_bytes, hit.tensor
 
 

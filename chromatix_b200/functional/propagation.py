@@ -251,10 +251,10 @@ def _pair_key(v):
 
 
 def _plan_key(field, zs, zshape, n, kykx, shift_yx, remove_evanescent, bandlimit, h_index):
-    dx = np.asarray(field.dx, dtype=np.float64)
-    return (type(field), dx.shape, dx.tobytes(), np.asarray(field.spectrum.wavelength, dtype=np.float64).tobytes(),
-            np.asarray(zs, dtype=np.float64).tobytes(), tuple(zshape), float(n), _pair_key(kykx), _pair_key(shift_yx),
-            bool(remove_evanescent), bool(bandlimit), None if h_index is None else np.asarray(h_index).tobytes())
+    dx, wl = np.asarray(field.dx, dtype=np.float64), field.spectrum.wavelength
+    return (type(field), dx.shape, dx.tobytes(), wl.dtype, wl.tobytes(), zs.dtype, zs.tobytes(), tuple(zshape), float(n),
+            _pair_key(kykx), _pair_key(shift_yx), bool(remove_evanescent), bool(bandlimit),
+            None if h_index is None else np.asarray(h_index).tobytes())
 
 
 class _GeneralPlan:
