@@ -98,6 +98,18 @@ __global__ void k_intensity(const float2* __restrict__ u, long n_pix, int W, con
   }
 }
 
+cx_status fft1d(const float2* in, float2* out, int n, long batch, bool inverse, const float2* twg, cudaStream_t st) {
+  switch (n) {
+#define CX_CASE_(N) \
+  case N:           \
+    return launch_fft1d<N>(in, out, batch, inverse, twg, st);
+    CX_FOR_EACH_1D_SIZE(CX_CASE_)
+#undef CX_CASE_
+  }
+  set_error("FFT length %d is not supported", n);
+  return CX_ERR_UNSUPPORTED;
+}
+
 }  // namespace cx
 
 using namespace cx;
@@ -118,18 +130,8 @@ extern "C" cx_status cx_fft1d(const void* in, void* out, int32_t n, int64_t batc
   const float2* twg = nullptr;
   cx_status s = ensure_twiddles(&twg);
   if (s != CX_OK) return s;
-  const float2* i = static_cast<const float2*>(in);
-  float2* o = static_cast<float2*>(out);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  switch (n) {
-#define CX_CASE_(N) \
-  case N:           \
-    return launch_fft1d<N>(i, o, batch, inverse != 0, twg, st);
-    CX_FOR_EACH_1D_SIZE(CX_CASE_)
-#undef CX_CASE_
-  }
-  set_error("FFT length %d is not supported", n);
-  return CX_ERR_UNSUPPORTED;
+  return fft1d(static_cast<const float2*>(in), static_cast<float2*>(out), n, batch, inverse != 0, twg,
+               static_cast<cudaStream_t>(stream));
 }
 
 extern "C" cx_status cx_intensity(const void* u, int64_t n_pix, int32_t n_wv, const double* density_dev, float* out,

@@ -116,7 +116,7 @@ extern "C" cx_status cx_czt(const cx_czt_desc* d, const void* x, void* y, void* 
   float2* chat = c + a.L;
   k_czt_filter<<<(a.L + 255) / 256, 256, 0, st>>>(c, a.n, a.m, a.L, a.tw, a.lw);
   CX_LAUNCH_CHECK();
-  if ((s = cx_fft1d(c, chat, a.L, 1, 0, stream)) != CX_OK) return s;
+  if ((s = fft1d(c, chat, a.L, 1, false, a.twg, st)) != CX_OK) return s;
   a.chat = chat;
   a.x = static_cast<const float2*>(x);
   a.y = static_cast<float2*>(y);
@@ -184,7 +184,7 @@ extern "C" cx_status cx_czt_noalloc(const cx_czt_desc* d, const void* x, void* y
   float2* chat = c + a.L;
   k_czt_filter<<<(a.L + 255) / 256, 256, 0, st>>>(c, a.n, a.m, a.L, a.tw, a.lw);
   CX_LAUNCH_CHECK();
-  if ((s = cx_fft1d(c, chat, a.L, 1, 0, stream)) != CX_OK) return s;
+  if ((s = fft1d(c, chat, a.L, 1, false, a.twg, st)) != CX_OK) return s;
   a.chat = chat;
   a.x = static_cast<const float2*>(x);
   a.y = static_cast<float2*>(y);

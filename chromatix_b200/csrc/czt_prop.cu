@@ -232,7 +232,7 @@ extern "C" cx_status cx_czt_propagate(const cx_czt_prop_desc* d, const void* u_i
       k_yu_filter<<<(Ls[k] + 255) / 256, 256, 0, st>>>(cfilt, Ls[k], cin, (double)(n - 1 - sc + n / 2), n - 1 - sc,
                                                        2 * n - 1 - sc);
       CX_LAUNCH_CHECK();
-      if ((s = cx_fft1d(cfilt, chat, Ls[k], 1, 0, stream)) != CX_OK) return s;
+      if ((s = fft1d(cfilt, chat, Ls[k], 1, false, twg, st)) != CX_OK) return s;
       CztArgs& a = yu[k];
       a.n = n;
       a.m = n;

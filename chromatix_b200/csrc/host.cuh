@@ -99,6 +99,9 @@ constexpr int kTwTotal = tw_total();
 // the propagations, optical FFTs, chirp-Z transforms and convolutions.
 cx_status ensure_twiddles(const float2** table, bool unit = false);
 
+// cx_fft1d with the given table (capi.cu).
+cx_status fft1d(const float2* in, float2* out, int n, long batch, bool inverse, const float2* twg, cudaStream_t st);
+
 // The real-expanded forward DFT matrices of the split-precision tensor-core
 // transforms (lengths 32 and 40): 2R x 2R, K-major canonical layout, FP16 hi
 // then lo, built on the host in FP64 and uploaded with the twiddle tables.
