@@ -291,8 +291,10 @@ def _pinned(arr: np.ndarray):
 def upload(arr: np.ndarray, device):
     """Host array -> device tensor through page-locked memory, asynchronous on
     the current stream: the host does not wait for the stream (a pageable
-    blocking copy would synchronise it, serialising host and device)."""
-    return _pinned(arr).to(device, non_blocking=True)
+    blocking copy would synchronise it, serialising host and device).  Not an
+    inference tensor: a copy that is kept may later be saved for a gradient."""
+    with torch_mod().inference_mode(False):
+        return _pinned(arr).to(device, non_blocking=True)
 
 
 class PlanCache:
