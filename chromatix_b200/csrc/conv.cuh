@@ -45,9 +45,6 @@ struct ConvArgs {
   int kh, kw;             // kernel (PSF) plane shape
   int HB;                 // rows per tile block of T: max(h, kh)
   int ldY;                // pair passes (conv_pair.cuh): rows of T's columns, HB rounded up to even
-  int slabs;              // CTAs that can share a column of the pair column pass; 1: at most two
-  int fresh;              // (slabs > 1) the first chunk: St holds nothing yet
-  float2* part;           // their partial sums (slabs, NC, P), where slabs > 1
   int NT, vt_shift;       // column tiles of T and their width VT = 1 << vt_shift (>= 4, a multiple of the column pass's V)
   int P, Q, M, NC;        // transform lengths, M = Q / 2, NC = M + 1
   int z0, zc;             // plane chunk
@@ -61,6 +58,9 @@ struct ConvArgs {
   int c0y, c0x;           // "same" crop offsets ((kh - 1) / 2, (kw - 1) / 2)
   float scale;            // 2 / (P Q)
   const float2* twg;
+  int slabs;              // CTAs that can share a column of the pair column pass; 1: at most two
+  int fresh;              // (slabs > 1) the first chunk: St holds nothing yet
+  float2* part;           // the shares' partial sums (slabs, NC, P), where slabs > 1
 };
 
 // ---------------------------------------------------------------------------

@@ -31,7 +31,6 @@ struct MsArgs {
   double lam, dz;
   float kdz_f;          // 2 pi dz / lam rounded once to float
   float kdz_lo;         // and what the rounding left
-  int rec_new;          // MS_BWD: rec_u comes from a recomputation that this launch follows
   int sy, sx, oy, ox;   // MS_LOAD source: (sy, sx) matrix placed at offset (oy, ox) of the padded grid
   const float* dn;      // (D, ny, nx) refractive-index change (unpadded)
   const float* ab;      // (D, ny, nx) absorption (unpadded)
@@ -46,6 +45,7 @@ struct MsArgs {
   const float* fl;      // MS_FLUOR: (D, ny, nx) fluorescence amplitude
   const float* ph;      // MS_FLUOR: (D, ny, nx) random phases
   float load_scale;     // MS_LOAD: factor on the source (1 / px when a row pass follows the load)
+  int rec_new;          // (for the launch) MS_BWD: rec_u comes from a recomputation that this launch follows
 };
 
 // thin-sample transmittance t = exp(i 2 pi dz / lam (dn + i abs))
