@@ -79,7 +79,7 @@ static cx_status conv_plan(const cx_conv_desc* d, ConvArgs* a, int* zc, size_t* 
   const int share = (ctas + a->NC - 1) / a->NC + 1;
   a->slabs = ctas <= a->NC || c <= 2 ? 1 : (share < c ? share : c);
   const size_t u_bytes = ((sizeof(float2) * (size_t)a->NC * d->h) + 255) & ~(size_t)255;
-  *total = *t_bytes + st_bytes + u_bytes + (a->slabs > 1 ? a->slabs * st_bytes : 0);
+  *total = kAlignSlack + *t_bytes + st_bytes + u_bytes + (a->slabs > 1 ? a->slabs * st_bytes : 0);
   return CX_OK;
 }
 
@@ -115,7 +115,7 @@ extern "C" cx_status cx_conv2d_same(const cx_conv_desc* d, const float* sample, 
   }
   if ((s = ensure_twiddles(&a.twg, true)) != CX_OK) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  char* ws = static_cast<char*>(workspace);
+  char* ws = align16(workspace);
   a.T = reinterpret_cast<float2*>(ws);
   a.St = reinterpret_cast<float2*>(ws + tb);
   a.U = reinterpret_cast<float2*>(ws + tb + (((sizeof(float2) * (size_t)a.NC * a.P) + 255) & ~(size_t)255));

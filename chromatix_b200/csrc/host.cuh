@@ -121,6 +121,13 @@ __device__ __forceinline__ void load_twiddles(float2* tw, const float2* __restri
 
 int sm_count();  // of the current device (capi.cu)
 
+// The first 16-byte boundary of a workspace whose query allows for kAlignSlack
+// more: the passes on pairs read and write row spectra 16 bytes at a time.
+constexpr size_t kAlignSlack = 16;
+inline char* align16(void* p) {
+  return reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(p) + 15) & ~static_cast<uintptr_t>(15));
+}
+
 // Register budget of the row / column kernels: about 80 registers per thread
 // (min blocks per SM derived from the CTA size).
 __host__ __device__ constexpr int minb_for(int threads) {

@@ -292,7 +292,7 @@ static size_t psf_cx_bytes(const cx_psf_desc* d) {
   return ((size_t)d->n_z * d->n_wv * d->nx * sizeof(float2) + 255) & ~(size_t)255;
 }
 static size_t psf_ws(const cx_psf_desc* d) {
-  return 256 + psf_t_bytes(d) + psf_m_bytes(d) + psf_cx_bytes(d) + sizeof(float2) * (size_t)d->n_z * d->n_wv * d->ny;
+  return kAlignSlack + 256 + psf_t_bytes(d) + psf_m_bytes(d) + psf_cx_bytes(d) + sizeof(float2) * (size_t)d->n_z * d->n_wv * d->ny;
 }
 
 }  // namespace cx
@@ -325,6 +325,7 @@ static cx_status psf_setup(const cx_psf_desc* d, const cx_psf_spectrum* spec, co
     set_error("workspace too small: %zu < %zu", workspace_bytes, psf_ws(d));
     return CX_ERR_WORKSPACE;
   }
+  workspace = align16(workspace);
   PsfArgs a = psf_make_args(d, spec, /*with_lens=*/true);
   a.z = z_dev;
   a.phase = phase;
@@ -371,8 +372,8 @@ static cx_status psf_setup(const cx_psf_desc* d, const cx_psf_spectrum* spec, co
   return CX_OK;
 }
 
-static cx_status psf_prepare(const PsfArgs& a, void* workspace, cudaStream_t st) {
-  CX_CUDA_TRY(cudaMemsetAsync(workspace, 0, 256, st));
+static cx_status psf_prepare(const PsfArgs& a, cudaStream_t st) {
+  CX_CUDA_TRY(cudaMemsetAsync(const_cast<unsigned long long*>(a.counts), 0, 256, st));
   k_psf_count<<<(a.W * a.ny + 127) / 128, 128, 0, st>>>(a, const_cast<unsigned long long*>(a.counts),
                                                          const_cast<int*>(a.srange));
   CX_LAUNCH_CHECK();
@@ -397,7 +398,7 @@ extern "C" cx_status cx_psf_4f(const cx_psf_desc* d, const cx_psf_spectrum* spec
   cx_status s = psf_setup(d, spec, z_dev, phase, intensity_out, workspace, workspace_bytes, &a, &zc);
   if (s != CX_OK) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if ((s = psf_prepare(a, workspace, st)) != CX_OK) return s;
+  if ((s = psf_prepare(a, st)) != CX_OK) return s;
   for (int z0 = 0; z0 < a.nz; z0 += zc) {
     a.z0 = z0;
     a.zc = (a.nz - z0) < zc ? (a.nz - z0) : zc;
@@ -436,7 +437,7 @@ extern "C" cx_status cx_psf_4f_stage(const cx_psf_desc* d, const cx_psf_spectrum
   cx_status s = psf_setup(d, spec, z_dev, phase, intensity_out, workspace, workspace_bytes, &a, &zc);
   if (s != CX_OK) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (stage < 0) return psf_prepare(a, workspace, st);
+  if (stage < 0) return psf_prepare(a, st);
   a.z0 = chunk * zc;
   if (a.z0 < 0 || a.z0 >= a.nz) {
     set_error("chunk %d out of range", chunk);
